@@ -114,6 +114,20 @@ ksim_status report_timeout(ksim_component *c)
 // Fill a SampleJob for component c; inputs/outputs set by the caller.
 ksim_status component_job(ksim_component *c, const LaunchCfg &cfg, SampleJob &j)
 {
+    j.n_graphs = c->img.n_graphs;
+    j.F = c->img.F;
+    j.n_out = c->img.n_out;
+    j.status = c->d_status;
+    j.wait_limit = c->wait_limit;
+    if (cfg.sliced) {
+        j.image = c->d_slices;
+        j.cdir = c->d_slice_dir;
+        j.n_chunks = c->slice_chunks;
+        j.slot_bytes = SLICE_SLOT;
+        j.s_rows = c->slice_rows;
+        j.s_planes = c->slice_planes;
+        return KSIM_OK;
+    }
     const ChunkDir *cd = nullptr;
     int nc = 0;
     const int slot = cfg.staged ? cfg.slot_bytes : (int)std::max<int64_t>(c->img.max_term_bytes, 16);
@@ -123,12 +137,7 @@ ksim_status component_job(ksim_component *c, const LaunchCfg &cfg, SampleJob &j)
     j.gdir = (const GraphDir *)c->d_image;
     j.cdir = cd;
     j.n_chunks = nc;
-    j.n_graphs = c->img.n_graphs;
-    j.F = c->img.F;
-    j.n_out = c->img.n_out;
     j.slot_bytes = slot;
-    j.status = c->d_status;
-    j.wait_limit = c->wait_limit;
     return KSIM_OK;
 }
 
@@ -197,6 +206,24 @@ ksim_status ksim_component_create(const ksim_graph_desc *graphs, int32_t n_graph
     c->image_bytes = c->img.bytes.size();
     e = cudaMemcpy(c->d_image, c->img.bytes.data(), c->img.bytes.size(), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpy(program image)");
+    SliceImage sl;
+    build_slices(graphs, c->img, sl);
+    if (sl.ok) {
+        const size_t at = (sl.bytes.size() + 31) & ~size_t(31);
+        sl.bytes.resize(at + sl.chunks.size() * sizeof(ChunkDir), 0);
+        std::memcpy(sl.bytes.data() + at, sl.chunks.data(), sl.chunks.size() * sizeof(ChunkDir));
+        e = cudaMalloc(&c->d_slices, sl.bytes.size());
+        if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(sliced stream)");
+        e = cudaMemcpy(c->d_slices, sl.bytes.data(), sl.bytes.size(), cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpy(sliced stream)");
+        c->d_slice_dir = (const ChunkDir *)(c->d_slices + at);
+        c->slice_chunks = (int)sl.chunks.size();
+        c->slice_rows = sl.rows;
+        c->slice_planes = sl.max_planes;
+        c->cfg.sliced = 1;
+        cudaDeviceGetAttribute(&c->cfg.sms, cudaDevAttrMultiProcessorCount, device);
+        c->image_bytes += sl.bytes.size();
+    }
     e = cudaMalloc(&c->d_status, sizeof(uint32_t));
     if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(status)");
     e = cudaMemset(c->d_status, 0, sizeof(uint32_t));
@@ -236,6 +263,7 @@ void ksim_component_destroy(ksim_component *c)
     c->ws_aux.release();
     if (c->d_status) cudaFree(c->d_status);
     if (c->d_image) cudaFree(c->d_image);
+    if (c->d_slices) cudaFree(c->d_slices);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
 }
@@ -255,6 +283,7 @@ ksim_status ksim_component_set_launch(ksim_component *c, int32_t threads, int32_
         if (threads > 256 || (threads & 31))
             return fail(KSIM_ERR_INVALID_ARGUMENT, "threads must be a multiple of 32 in [32, 256]");
         cfg.threads = threads;
+        cfg.slice_threads = threads;
     }
     if (staged >= 0) cfg.staged = staged ? 1 : 0;
     if (slot_bytes > 0) {

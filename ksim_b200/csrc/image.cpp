@@ -214,6 +214,7 @@ int build_image(const ksim_graph_desc *gs, int n_graphs, int F, HostImage &img, 
     img.W = W;
     img.gdir.resize(n_graphs);
     img.term_off.resize(n_graphs);
+    img.term_proof.resize(n_graphs);
     std::vector<uint8_t> &out = img.bytes;
     out.resize(sizeof(GraphDir) * (size_t)n_graphs, 0);
 
@@ -665,7 +666,7 @@ int build_image(const ksim_graph_desc *gs, int n_graphs, int F, HostImage &img, 
                 if (rows.size() > (size_t)32 * NB_MAX) unsafe = true;
             }
             if (unsafe) flags = TF_SLOW;
-            if (!unsafe) {
+            {
                 // the scales 2^(pw + power2) a shot can reach: pw starts at
                 // H or at a kill's dead_pw and gains at most two halvings per
                 // PhasePairs pair and one renormalisation
@@ -677,7 +678,9 @@ int build_image(const ksim_graph_desc *gs, int n_graphs, int F, HostImage &img, 
                     }
                 hi += 2 * (int64_t)((n_ph + 1) / 2) + 1;
                 const int64_t p2 = g.pf_power2[t];
-                if (p2 + lo >= -1022 && p2 + hi <= 1023) flags |= TF_EXP;
+                const bool normal = p2 + lo >= -1022 && p2 + hi <= 1023;
+                if (!unsafe && normal) flags |= TF_EXP;
+                img.term_proof[k].push_back((uint8_t)((ref_max <= kLim ? TP_REF : 0) | (normal ? TP_SCALE : 0)));
             }
             if (g.pf_has_approx) flags |= TF_APX;
             std::vector<uint8_t> body;  // everything after the header (and approximation)

@@ -28,11 +28,16 @@ static_assert(sizeof(ChunkDir) == 32, "ChunkDir layout");
 // Supported parameter-vector widths (64-bit words); images are padded up to one.
 int supported_words(int needed);
 
+// What the packer proved about a term: the reference's int64 arithmetic cannot
+// wrap; every scale 2^(pw + power2) it can reach is a normal double.
+enum : uint8_t { TP_REF = 1, TP_SCALE = 2, TP_ALL = 3 };
+
 struct HostImage {
     int n_graphs = 0, F = 0, n_out = 0, W = 0;
     std::vector<uint8_t> bytes;                  // [GraphDir x n_graphs][term streams]
     std::vector<GraphDir> gdir;
     std::vector<std::vector<int64_t>> term_off;  // per graph: term start offsets + end
+    std::vector<std::vector<uint8_t>> term_proof;  // per graph and term: TP_* bits
     int64_t max_term_bytes = 0;
     int64_t n_terms = 0, n_slow_terms = 0, n_narrow_terms = 0, n_hybrid_terms = 0;
     double work_ops = 0;  // int32 operations per shot, all graphs (term_work / graph_work)

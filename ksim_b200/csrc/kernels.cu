@@ -12,6 +12,7 @@
 #include "../../include/ksim_b200.h"
 #include "kernels.h"
 #include "sample_tile.cuh"
+#include "slice_tile.cuh"
 #include "zring.cuh"
 
 namespace ksim {
@@ -34,6 +35,21 @@ __global__ void KSIM_SAMPLE_BOUNDS(PATHS) k_sample(const SampleJob j)
     uint8_t *scratch = STAGED ? slots + (size_t)NSLOT * j.slot_bytes : slots;
     sample_tile<W, STAGED, false, S, PATHS>(j, (int64_t)blockIdx.x * blockDim.x * S, bar, slots, g,
                                                    scratch);
+}
+
+// The sliced sampler: one CTA per `tile` shots (tile <= shots, the width of
+// the CTA's bit rows).  S shots a thread; THREADS and CTAS bound the registers.
+template <int S, int THREADS, int CTAS>
+__global__ void __launch_bounds__(THREADS, CTAS) k_slice(const SampleJob j, const int shots, const int tile)
+{
+    extern __shared__ __align__(128) uint8_t smem[];
+    uint8_t *ring = smem + slice_ring_off(j.s_rows, j.s_planes, shots);
+    uint64_t *bar = (uint64_t *)ring;
+    ring_init(bar);
+    uint32_t g = 0;
+    const int64_t s0 = (int64_t)blockIdx.x * tile;
+    slice_tile<S>(j, s0, s0 + tile < j.B ? s0 + tile : j.B, shots, smem, slice_rows_bytes(j.s_rows, shots), bar,
+                  ring + BAR_BYTES, g);
 }
 
 template <int W>
@@ -113,6 +129,51 @@ cudaError_t launch_sample_w(const SampleJob &j, const LaunchCfg &cfg, cudaStream
     return cudaGetLastError();
 }
 
+template <int S, int THREADS, int CTAS>
+cudaError_t launch_slice_as(const SampleJob &j, int shots, int threads, int tile, cudaStream_t st)
+{
+    const int64_t blocks = (j.B + tile - 1) / tile;
+    if (blocks > 0x7FFFFFFF) return cudaErrorInvalidConfiguration;
+    const int smem = slice_smem_bytes(j.s_rows, j.s_planes, shots);
+    cudaError_t e = cudaFuncSetAttribute(k_slice<S, THREADS, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    k_slice<S, THREADS, CTAS><<<(unsigned)blocks, threads, smem, st>>>(j, shots, tile);
+    return cudaGetLastError();
+}
+
+// The tile shape by how many SMs the shots can fill.  Measured on the 40-output
+// t = 12 program (ms; 512 threads x 1 shot at widths 128 / 256 / 512, 512 x 2
+// at 1,024 -- 256 threads x 4, two CTAs an SM -- 256 x 8 at 2,048, two CTAs):
+//    10,000 shots  0.236 0.249 0.267 0.36 0.41 0.68    (19,000 = 148 x 128)
+//    20,000        0.42  0.247 0.269 0.36 0.41 0.68
+//    70,000        0.85  0.49  0.271 0.36 0.41 0.68
+//   100,000        1.26  0.66  0.53  0.363 0.415 0.68
+//   200,000              1.1   0.79  0.72 0.547 0.68   (303,104 = 296 x 1,024)
+//   500,000                    1.84  1.43 1.08 0.92
+// and alike on the 16-output t = 20 one: the widest tile costs least per shot,
+// but a narrower one that still fits one wave ends sooner.
+cudaError_t launch_slice(const SampleJob &j, const LaunchCfg &cfg, cudaStream_t st)
+{
+    if (cfg.slice_threads > 0) {  // threads chosen by the caller: four shots each
+        const int t = cfg.slice_threads >= 256 ? 256 : cfg.slice_threads >= 128 ? 128 : cfg.slice_threads >= 64 ? 64 : 32;
+        return launch_slice_as<4, 256, 2>(j, 4 * t, t, 4 * t, st);
+    }
+    const int64_t sms = cfg.sms;
+    if (j.B <= sms * 512) {
+        const int shots = j.B <= sms * 128 ? 128 : j.B <= sms * 256 ? 256 : 512;
+        return launch_slice_as<1, 512, 1>(j, shots, 512, shots, st);
+    }
+    if (j.B <= sms * 1024) return launch_slice_as<4, 512, 1>(j, 1024, 512, 1024, st);
+    const bool wide = j.B > 2 * sms * 1024;
+    const int shots = wide ? 2048 : 1024;
+    // equal tiles: a last wave that is nearly empty costs as much as a full one
+    const int64_t waves = (j.B + 2 * sms * shots - 1) / (2 * sms * shots);
+    const int64_t want = (j.B + waves * 2 * sms - 1) / (waves * 2 * sms);
+    const int tile = (int)((want + 63) / 64 * 64);
+    if (wide) return launch_slice_as<8, 256, 2>(j, shots, 256, tile, st);
+    return launch_slice_as<4, 256, 2>(j, shots, 256, tile, st);
+}
+
 template <int W>
 cudaError_t launch_eval_w(const EvalJob &j, cudaStream_t st)
 {
@@ -183,6 +244,7 @@ cudaError_t launch_sample(const SampleJob &job, int W, const LaunchCfg &cfg, cud
 {
     if (job.B <= 0) return cudaSuccess;
     if (cfg.threads <= 0 || cfg.threads > 256 || (cfg.threads & 31)) return cudaErrorInvalidConfiguration;
+    if (cfg.sliced) return launch_slice(job, cfg, st);
     switch (W) {
     case 1: return launch_sample_w<1>(job, cfg, st);
     case 2: return launch_sample_w<2>(job, cfg, st);

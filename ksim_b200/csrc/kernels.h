@@ -51,13 +51,16 @@ struct SampleJob {
     uint64_t seed;
     uint32_t *status;          // KSIM_FLAG_* accumulator
     int64_t wait_limit;        // > 0: a staging wait gives up after this many test_wait polls
-    int64_t reserved;
+    int32_t s_rows, s_planes;  // sliced stream (image, cdir and n_chunks are its): parameter rows, result planes
 };
 
 struct LaunchCfg {
     int threads = 256;   // shots per CTA (one shot per thread)
     int staged = 1;      // stage term chunks in shared memory with TMA bulk copies
     int slot_bytes = 16384;
+    int sliced = 0;         // run the sliced stream (its own staging)
+    int slice_threads = 0;  // its threads per CTA (0: tile shape from the shots)
+    int sms = 148;          // SMs of the device
     int paths = 0;       // term paths the program uses: 0 all, 1 32-bit only, 2 32-bit and hybrid
                          // (the kernels compiled without the others)
 };

@@ -11,6 +11,7 @@
 #include "../../include/ksim_b200.h"
 #include "image.h"
 #include "kernels.h"
+#include "slice.h"
 
 namespace ksim {
 
@@ -46,6 +47,11 @@ struct ksim_component {
     uint8_t *d_image = nullptr;
     size_t image_bytes = 0;
     std::map<int, ksim::ComponentChunks> chunks;  // by staging slot size
+    // the sliced stream (slice.h): [chunks and tables][chunk directory]; null
+    // when a term does not qualify
+    uint8_t *d_slices = nullptr;
+    const ksim::ChunkDir *d_slice_dir = nullptr;
+    int slice_chunks = 0, slice_rows = 0, slice_planes = 0;
     uint32_t *d_status = nullptr;
     cudaStream_t stream = nullptr;
     ksim::DevBuf ws_f, ws_out, ws_aux;

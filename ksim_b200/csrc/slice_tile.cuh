@@ -1,0 +1,619 @@
+// slice_tile.cuh — the per-CTA sampling loop over a sliced stream (slice.h).
+//
+// The parameter vector of a tile's shots lives bit-sliced in shared memory:
+// one row of words per parameter, bit = shot.  Per chunk of terms the CTA
+// runs two passes:
+//   rows    a warp takes one half of a term (its K roles or its X roles): L
+//           lanes cover the tile's shots, 64 each, and the 32 / L lane groups
+//           share the quads of every role.  A lane forms parity rows as XORs
+//           of a few parameter words and adds them into bit-sliced counters
+//           (carry-save adders); the groups' counters are added over
+//           shuffles, and the eight result planes become one byte per shot by
+//           in-register 8 x 8 bit transposes;
+//   values  a thread takes its S shots: two result bytes a term give the
+//           table entry (a complex double), its rotation by i^k and whether
+//           the term is dead; the entries are added in term order.
+// At a graph's end each thread makes its Bernoulli draws and the warp writes
+// the sampled output's row with ballots (kokkos_sim.cpp:214-230).
+//
+// Chunks are staged by TMA bulk copies in a two-slot ring as in
+// sample_tile.cuh, with the same bounded waits.
+#pragma once
+#include "sample_tile.cuh"
+#include "slice.h"
+
+namespace ksim {
+
+// Shared memory of a sliced tile of `shots` (64 to 2,048, a power of two):
+// parameter rows, result planes, then the barriers and the ring.
+// (The rows of a 2,048-shot tile are two regions, 1,024 shots each.)
+__host__ __device__ constexpr int slice_region(int rows) { return (rows + 1) * SLICE_ROW; }
+__host__ __device__ constexpr int slice_rows_bytes(int rows, int shots)
+{
+    return slice_region(rows) * (shots > 1024 ? 2 : 1);
+}
+__host__ __device__ constexpr int slice_ring_off(int rows, int planes, int shots)
+{
+    return (slice_rows_bytes(rows, shots) + planes * shots + 127) & ~127;
+}
+__host__ __device__ constexpr int slice_smem_bytes(int rows, int planes, int shots)
+{
+    return slice_ring_off(rows, planes, shots) + BAR_BYTES + NSLOT * SLICE_SLOT;
+}
+
+struct W2 {
+    uint32_t a, b;
+};
+__device__ __forceinline__ W2 operator^(W2 x, W2 y) { return {x.a ^ y.a, x.b ^ y.b}; }
+__device__ __forceinline__ W2 operator&(W2 x, W2 y) { return {x.a & y.a, x.b & y.b}; }
+__device__ __forceinline__ W2 operator|(W2 x, W2 y) { return {x.a | y.a, x.b | y.b}; }
+__device__ __forceinline__ W2 operator~(W2 x) { return {~x.a, ~x.b}; }
+__device__ __forceinline__ W2 maj(W2 x, W2 y, W2 z)
+{
+    return {(x.a & y.a) | (x.a & z.a) | (y.a & z.a), (x.b & y.b) | (x.b & z.b) | (y.b & z.b)};
+}
+
+// The N rows of a group for this lane's 64 shots.  lane8: the shared address
+// of the lane's column of the parameter rows.  A slot's address is one dot
+// product (byte k of the word times the row pitch, plus the column).
+template <int N>
+__device__ __forceinline__ void slice_rows(uint32_t entry, const uint8_t *chunk, uint32_t lane8, W2 (&r)[N])
+{
+    const uint4 *p = (const uint4 *)(chunk + 16u * (entry & 0xFFFFu));
+    int n = (int)((entry >> 16) & 0xFFu);
+    uint32_t u[N];
+    auto words = [&](uint32_t (&x)[N]) {
+#pragma unroll
+        for (int i = 0; i < N; i += 4) {
+            const uint4 v = *p++;
+            x[i] = v.x; x[i + 1] = v.y; x[i + 2] = v.z; x[i + 3] = v.w;
+        }
+    };
+    words(u);
+#pragma unroll
+    for (int i = 0; i < N; ++i) r[i] = {u[i], u[i]};
+    words(u);
+    auto ld = [&](uint32_t x, int k) {
+        W2 v;
+        asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.a), "=r"(v.b)
+                     : "r"(__dp4a(x, (uint32_t)SLICE_ROW << (8 * k), lane8)));
+        return v;
+    };
+    auto one = [&](int k) {
+        W2 x[N];
+#pragma unroll
+        for (int i = 0; i < N; ++i) x[i] = ld(u[i], k);
+#pragma unroll
+        for (int i = 0; i < N; ++i) r[i] = r[i] ^ x[i];
+    };
+    auto two = [&](int k) {
+#pragma unroll
+        for (int h = 0; h < N; h += 4) {
+            W2 x[4], y[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = ld(u[h + i], k);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) y[i] = ld(u[h + i], k + 1);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) r[h + i] = r[h + i] ^ x[i] ^ y[i];
+        }
+    };
+    for (;;) {
+        if (n == 1) {
+            one(0);
+            break;
+        }
+        two(0);
+        if (n == 2) break;
+        if (n == 3) {
+            one(2);
+            break;
+        }
+        two(2);
+        n -= 4;
+        if (n == 0) break;
+        words(u);
+    }
+}
+
+__device__ __forceinline__ W2 slice_shfl(W2 x, int o)
+{
+    return {__shfl_xor_sync(~0u, x.a, o), __shfl_xor_sync(~0u, x.b, o)};
+}
+
+// Add the counters (planes FROM..TO - 1) of lane groups o lanes apart.
+template <int FROM, int TO, int N>
+__device__ __forceinline__ void slice_add(W2 (&c)[N], int o)
+{
+    W2 carry = {0u, 0u};
+#pragma unroll
+    for (int i = FROM; i < TO; ++i) {
+        const W2 x = slice_shfl(c[i], o), t = maj(c[i], x, carry);
+        c[i] = c[i] ^ x ^ carry;
+        carry = t;
+    }
+}
+
+// Eight planes of 32 shots to 32 bytes: word r, byte j of q holds bit 8 j + r
+// of every plane, plane k in its bit k.  Stored as the 32 bytes at o.
+__device__ __forceinline__ void slice_store(uint32_t (&p)[8], uint8_t *o)
+{
+#pragma unroll
+    for (int d = 4; d >= 1; d >>= 1) {
+        const uint32_t m = d == 4 ? 0x0F0F0F0Fu : d == 2 ? 0x33333333u : 0x55555555u;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (i & d) continue;
+            const uint32_t x = p[i], y = p[i + d];
+            p[i] = (x & m) | ((y << d) & ~m);
+            p[i + d] = ((x >> d) & m) | (y & ~m);
+        }
+    }
+    ((uint4 *)o)[0] = make_uint4(p[0], p[1], p[2], p[3]);
+    ((uint4 *)o)[1] = make_uint4(p[4], p[5], p[6], p[7]);
+}
+
+// The warp's place in a rows pass: L lanes a group, this lane's group and its
+// column.  The result words li and li + L are stored by the first two groups,
+// or both by the only one.
+struct SliceLane {
+    int L, li, grp, n_grp;
+    uint32_t lane8;
+};
+template <typename F>
+__device__ __forceinline__ void slice_finish(const SliceLane &ln, F &&store)
+{
+    if (ln.grp > 1) return;
+    int h = ln.grp;
+    for (;;) {
+        store(h, ln.li + h * ln.L);
+        if (ln.n_grp > 1 || h) break;
+        h = 1;
+    }
+}
+__device__ __forceinline__ uint32_t slice_pick(W2 x, int h) { return h ? x.b : x.a; }
+
+// x += b0 + ... + b3 in planes of weight 1, 2 (carries of weight 4 returned).
+__device__ __forceinline__ W2 slice_add4(W2 &x0, W2 &x1, W2 b0, W2 b1, W2 b2, W2 b3)
+{
+    const W2 t0 = maj(x0, b0, b1);
+    x0 = x0 ^ b0 ^ b1;
+    const W2 t1 = maj(x0, b2, b3);
+    x0 = x0 ^ b2 ^ b3;
+    const W2 f = maj(x1, t0, t1);
+    x1 = x1 ^ t0 ^ t1;
+    return f;
+}
+// The same into one plane, the carries xored into the next.
+__device__ __forceinline__ void slice_add4x(W2 &x0, W2 &x1, W2 b0, W2 b1, W2 b2, W2 b3)
+{
+    const W2 t0 = maj(x0, b0, b1);
+    x0 = x0 ^ b0 ^ b1;
+    const W2 t1 = maj(x0, b2, b3);
+    x0 = x0 ^ b2 ^ b3;
+    x1 = x1 ^ t0 ^ t1;
+}
+
+// One half of a term.  Planes a[]: K half 0-2 K, 3 kill, 4-7 y, 8-11 z; X half
+// 0-6 X, 7 S.  One loop over the half's groups, so the row code exists once.
+__device__ __forceinline__ void slice_task(const uint8_t *chunk, const SliceTerm &d, bool x_half, uint8_t *planes,
+                                           int plane_bytes, const SliceLane &ln)
+{
+    const uint32_t *list = (const uint32_t *)(chunk + 16 * (int)d.list_off16) + (x_half ? (int)d.n_k : 0);
+    const int n = x_half ? d.n_x : d.n_k;
+    W2 a[12];
+#pragma unroll
+    for (int i = 0; i < 12; ++i) a[i] = {0u, 0u};
+    bool n9 = false;
+    for (int q = ln.grp; q < n; q += ln.n_grp) {
+        const uint32_t e = list[q], role = (e >> 24) & 15u;
+        W2 r[SLICE_GROUP];
+        slice_rows<SLICE_GROUP>(e, chunk, ln.lane8, r);
+        if (role == SQ_X1 || role == SQ_X0) {
+            if (role == SQ_X1) {
+#pragma unroll
+                for (int i = 0; i < SLICE_GROUP; i += 2) a[7] = a[7] ^ r[i] ^ r[i + 1];
+            }
+            W2 c = slice_add4(a[0], a[1], r[0], r[1], r[2], r[3]);
+            int from = 2;
+            if (SLICE_GROUP == 8) {
+                const W2 f = slice_add4(a[0], a[1], r[SLICE_GROUP - 4], r[SLICE_GROUP - 3], r[SLICE_GROUP - 2], r[SLICE_GROUP - 1]);
+                const W2 t = maj(a[2], c, f);
+                a[2] = a[2] ^ c ^ f;
+                c = t;
+                from = 3;
+            }
+#pragma unroll
+            for (int i = 2; i < 7; ++i) {
+                if (i < from) continue;
+                const W2 t = a[i] & c;
+                a[i] = a[i] ^ c;
+                c = t;
+            }
+        } else if (role == SQ_PPX || role == SQ_PPK) {
+            W2 t = (r[0] & r[1]) ^ (r[2] & r[3]);
+#pragma unroll
+            for (int i = 4; i < SLICE_GROUP; i += 2) t = t ^ (r[i] & r[i + 1]);
+            if (role == SQ_PPX) a[7] = a[7] ^ t;
+            else a[2] = a[2] ^ t;
+        } else if (role == SQ_W2) {
+#pragma unroll
+            for (int i = 0; i < SLICE_GROUP; i += 4) slice_add4x(a[1], a[2], r[i], r[i + 1], r[i + 2], r[i + 3]);
+        } else if (role == SQ_W4) {
+#pragma unroll
+            for (int i = 0; i < SLICE_GROUP; i += 2) a[2] = a[2] ^ r[i] ^ r[i + 1];
+        } else if (role == SQ_KILL) {
+#pragma unroll
+            for (int i = 0; i < SLICE_GROUP; i += 2) a[3] = a[3] | r[i] | r[i + 1];
+        } else if (role == SQ_W1) {
+#pragma unroll
+            for (int i = 0; i < SLICE_GROUP; i += 4)
+                a[2] = a[2] ^ slice_add4(a[0], a[1], r[i], r[i + 1], r[i + 2], r[i + 3]);
+        } else {  // SQ_N9
+            n9 = true;
+#pragma unroll
+            for (int i = 0; i < SLICE_GROUP; i += 2) {
+                W2 yb = ~(r[i] | r[i + 1]), zb = r[i] & r[i + 1];
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    const W2 ty = a[4 + b] & yb, tz = a[8 + b] & zb;
+                    a[4 + b] = a[4 + b] ^ yb;
+                    a[8 + b] = a[8 + b] ^ zb;
+                    yb = ty;
+                    zb = tz;
+                }
+            }
+        }
+    }
+    n9 = __any_sync(~0u, n9);
+    for (int o = ln.L; o < 32; o <<= 1) {
+        if (x_half) {
+            a[7] = a[7] ^ slice_shfl(a[7], o);
+            slice_add<0, 7>(a, o);
+        } else {
+            a[3] = a[3] | slice_shfl(a[3], o);
+            slice_add<0, 3>(a, o);
+            if (n9) {
+                slice_add<4, 8>(a, o);
+                slice_add<8, 12>(a, o);
+            }
+        }
+    }
+    uint8_t *out = planes + ((int)d.plane + (x_half ? 0 : 1)) * plane_bytes;
+    const bool even = d.flags & ST_EVEN, wide = d.flags & ST_WIDE;
+    slice_finish(ln, [&](int h, int word) {
+        uint32_t p[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) p[i] = slice_pick(a[i], h);
+        if (!x_half) {
+            const uint32_t k0 = p[0], k1 = p[1], k2 = p[2], kill = p[3];
+            const uint32_t y0 = p[4], y1 = p[5], y2 = p[6], z0 = slice_pick(a[8], h), z1 = slice_pick(a[9], h),
+                           z2 = slice_pick(a[10], h);
+            if (wide) {
+                uint32_t w[8] = {y0, y1, y2, p[7], z0, z1, z2, slice_pick(a[11], h)};
+                slice_store(w, out + plane_bytes + 32 * word);
+            }
+            // class e (e + 1) / 2 + z, e = y + z <= 4 (ST_WIDE: 0)
+            const uint32_t on = wide ? 0u : ~0u;
+            const uint32_t e0 = y0 ^ z0, c0 = y0 & z0, e1 = y1 ^ z1 ^ c0;
+            const uint32_t e2 = (y2 | z2 | (y1 & z1) | (y1 & c0) | (z1 & c0)) & on;
+            const uint32_t t0 = (e0 ^ e1) & on, t1 = (e1 | e2) & on, t2 = e0 & e1 & on;  // e (e + 1) / 2; its bit 3 is e2
+            const uint32_t w0 = z0 & on, w1 = z1 & on, w2 = z2 & on;
+            const uint32_t q0 = t0 & w0, q1 = (t1 & w1) | (t1 & q0) | (w1 & q0), q2 = (t2 & w2) | (t2 & q1) | (w2 & q1);
+            const uint32_t cl0 = t0 ^ w0, cl1 = t1 ^ w1 ^ q0, cl2 = t2 ^ w2 ^ q1, cl3 = e2 ^ q2;
+            p[0] = k1;
+            p[1] = even ? cl0 : k0;
+            p[2] = even ? cl1 : cl0;
+            p[3] = even ? cl2 : cl1;
+            p[4] = even ? cl3 : cl2;
+            p[5] = even ? 0u : cl3;
+            p[6] = kill;
+            p[7] = k2;
+        }
+        slice_store(p, out + 32 * word);
+    });
+}
+
+// u < rn(mag / prev), the draw of kokkos_sim.cpp:226-227, without the division
+// where the product u * prev is clear of mag: t = rn(u prev) is within 2^-53
+// of it relatively (normal t), so outside t (1 +- 2^-50) the quotient's
+// rounding cannot change the comparison.  Everything else (and NaN, zeros,
+// infinities beside infinities) divides.  flags: KSIM_FLAG_* raised.
+__device__ __noinline__ double slice_philox(uint64_t seed, uint64_t shot, uint32_t output)
+{
+    return philox_uniform(seed, shot, output);
+}
+__device__ __noinline__ uint32_t slice_draw_exact(double u, double mag, double prev)
+{
+    const double ratio = __ddiv_rn(mag, prev);
+    return (u < ratio ? 1u : 0u) | (!(prev > 0.0) ? (uint32_t)KSIM_FLAG_PREV_NONPOSITIVE << 8 : 0u) |
+           (ratio != ratio ? (uint32_t)KSIM_FLAG_NAN << 8 : 0u);
+}
+__device__ __forceinline__ bool slice_draw(double u, double mag, double prev, uint32_t &flags)
+{
+    const double t = dmul(u, prev);
+    bool bit = mag > dmul(t, 1.0 + 0x1p-50);
+    if (!(t > 0x1p-900) || !(bit || mag < dmul(t, 1.0 - 0x1p-50))) {
+        const uint32_t x = slice_draw_exact(u, mag, prev);
+        bit = x & 1u;
+        flags |= x >> 8;
+    }
+    return bit;
+}
+
+// xorshift_uniform with the 53-bit integer converted through two exact
+// doubles (2^84 + hi 2^32, 2^52 + lo) instead of a 64-bit conversion.
+__device__ __forceinline__ double slice_xorshift(uint64_t &s)
+{
+    s ^= s << 13;
+    s ^= s >> 7;
+    s ^= s << 17;
+    const uint64_t v = s >> 11;
+    const double h = __hiloint2double(0x45300000, (int)(uint32_t)(v >> 32));
+    const double l = __hiloint2double(0x43300000, (int)(uint32_t)v);
+    return dmul(dadd(dsub(h, 0x1p84), dsub(l, 0x1p52)), 0x1p-53);
+}
+
+__device__ __forceinline__ uint32_t byte_of(uint32_t x, int k) { return (x >> (8 * k)) & 0xFFu; }
+
+// A thread's bytes of a result plane.
+template <int N>
+__device__ __forceinline__ uint32_t slice_plane(const uint8_t *p)
+{
+    return N == 4 ? *(const uint32_t *)p : *p;
+}
+
+// Issue the copy of a chunk (`bytes` at `off` of the job's stream) as the
+// gidx-th of the CTA.
+__device__ __forceinline__ void slice_issue(const SampleJob &j, int64_t off, uint32_t bytes, uint32_t gidx,
+                                            uint64_t *bar, uint8_t *slots)
+{
+    const int slot = (int)(gidx & (NSLOT - 1));
+    mbar_arrive_expect_tx(&bar[slot], bytes);
+    tma_bulk_g2s(slots + (size_t)slot * SLICE_SLOT, j.image + off, bytes, &bar[slot]);
+}
+
+// Sample shots [s0, s_end) of job j in a tile of `shots`, S of them a thread
+// (shots / S threads; the others only share the rows pass).  smem: the CTA's shared
+// memory, parameter rows first, planes at planes_off.  Returns false after a
+// wait timeout (the CTA must then stop using the ring).
+template <int S, bool CG = false>
+__device__ __forceinline__ bool slice_tile(const SampleJob &j, const int64_t s0, const int64_t s_end, int shots,
+                                           uint8_t *smem, int planes_off, uint64_t *bar, uint8_t *slots, uint32_t &g)
+{
+    static_assert(S == 1 || S == 4 || S == 8, "shots per thread");
+    const int tid = threadIdx.x, lane = tid & 31, nthr = (int)blockDim.x;
+    uint8_t *planes = smem + planes_off;
+    const int plane_bytes = shots;
+    const int F = j.F, R = j.s_rows;
+    const int region = slice_region(R);
+    SliceLane ln;
+    ln.L = shots >> 6;
+    ln.li = lane & (ln.L - 1);
+    ln.grp = lane / ln.L;
+    ln.n_grp = 32 / ln.L;
+    ln.lane8 = smem_u32(smem) + 8u * (uint32_t)(ln.li & 15) + (uint32_t)((ln.li >> 4) * region);
+    // this thread's shots: bits sh_bit(0), ... of word w (32 shots)
+    //   S = 8: bits r + 8 k and r + 4 + 8 k;  S = 4: bits r + 8 k;  S = 1: bit r
+    const bool mine = tid * S < shots;
+    const int w = tid * S >> 5, r = S == 8 ? tid & 3 : S == 4 ? tid & 7 : lane;
+    const int64_t sh0 = s0 + 32 * w + r;
+    auto sh_of = [&](int k) { return sh0 + (S == 8 ? 8 * (k & 3) + 4 * (k >> 2) : 8 * k); };
+    // its bytes of a result plane: word r of the 32 (and r + 4), or one byte
+    const int byte0 = S == 1 ? 32 * w + 4 * (lane & 7) + (lane >> 3) : 32 * w + 4 * r;
+    uint32_t act = 0;
+#pragma unroll
+    for (int k = 0; k < S; ++k) act |= mine && sh_of(k) < s_end ? 1u << k : 0u;
+    const bool warp_any = __any_sync(~0u, act != 0);
+    // word w of a parameter row: lane w mod L's 64-bit column
+    const int wl = w & (ln.L - 1);
+    const int wcol = (wl & 15) * 8 + (wl >> 4) * region + (w >= ln.L ? 4 : 0);
+    auto put_row = [&](int row, const bool (&x)[S]) {
+        uint32_t b[S];
+#pragma unroll
+        for (int k = 0; k < S; ++k) b[k] = __ballot_sync(~0u, x[k]);
+        uint8_t *o = smem + row * SLICE_ROW + wcol;
+        if (S == 8) {  // byte r of the word: the word's nibble of ballots r and r + 4
+            const uint32_t lo = r & 2 ? (r & 1 ? b[3 % S] : b[2 % S]) : (r & 1 ? b[1 % S] : b[0]);
+            const uint32_t hi = r & 2 ? (r & 1 ? b[7 % S] : b[6 % S]) : (r & 1 ? b[5 % S] : b[4 % S]);
+            const int sh = 4 * (w & 7);
+            if (mine) o[r] = (uint8_t)(((lo >> sh) & 15u) | ((hi >> sh) & 15u) << 4);
+        } else if (S == 4) {  // byte w & 3 of each ballot
+            const uint32_t sel = (uint32_t)(w & 3) | ((uint32_t)(4 + (w & 3)) << 4);
+            const uint32_t x0 = __byte_perm(b[0], b[1 % S], sel), x1 = __byte_perm(b[2 % S], b[3 % S], sel);
+            if (mine && r == 0) *(uint32_t *)o = __byte_perm(x0, x1, 0x5410);
+        } else {
+            if (mine && r == 0) *(uint32_t *)o = b[0];
+        }
+    };
+
+    // parameter rows: the f bits (four bytes at a time where rows allow it),
+    // outputs zero for graph 0, the zero row
+    const bool vec = !j.f_sel && ((((uintptr_t)j.f) | (uintptr_t)j.f_stride) & 3u) == 0;
+    int p0 = 0;
+    if (vec) {
+        for (; p0 + 8 <= F; p0 += 8) {
+            uint32_t x[S][2];
+#pragma unroll
+            for (int k = 0; k < S; ++k)
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    x[k][h] = ((act >> k) & 1u)
+                                  ? ldj<CG>((const uint32_t *)(j.f + sh_of(k) * j.f_stride + p0) + h) : 0u;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                bool b[S];
+#pragma unroll
+                for (int k = 0; k < S; ++k) b[k] = x[k][i >> 2] & (1u << (8 * (i & 3)));
+                put_row(p0 + i, b);
+            }
+        }
+    }
+    for (; p0 < F; p0 += 4) {
+        uint8_t x[S][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int p = min(p0 + i, F - 1);
+            const int col = j.f_sel ? ldj<CG>(j.f_sel + p) : p;
+#pragma unroll
+            for (int k = 0; k < S; ++k)
+                x[k][i] = ((act >> k) & 1u) ? ldj<CG>(j.f + sh_of(k) * j.f_stride + col) : (uint8_t)0;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            bool b[S];
+#pragma unroll
+            for (int k = 0; k < S; ++k) b[k] = x[k][i] & 1u;
+            if (p0 + i < F) put_row(p0 + i, b);
+        }
+    }
+    auto fill_rows = [&](int from, int to, uint32_t x) {
+        for (int i = tid; i < (to - from) * (SLICE_ROW / 4); i += nthr) {
+            ((uint32_t *)(smem + from * SLICE_ROW))[i] = x;
+            if (ln.L > 16) ((uint32_t *)(smem + region + from * SLICE_ROW))[i] = x;
+        }
+    };
+    fill_rows(F, R + 1, 0u);
+
+    uint64_t rng[S];
+    double prev[S], sre[S], sim[S];
+#pragma unroll
+    for (int k = 0; k < S; ++k) {
+        rng[k] = xorshift_init(j.seed, (uint64_t)(j.shot_offset + sh_of(k)));
+        prev[k] = 0.0;
+        sre[k] = 0.0;
+        sim[k] = 0.0;
+    }
+    uint32_t flags = 0, idle_flags = 0;  // (idle: shots past the job's end)
+    const int nch = j.n_chunks;
+    __syncthreads();
+    if (tid == 0)
+        for (int c = 0; c < NSLOT && c < nch; ++c) {
+            const ChunkDir d = ld_chunk<CG>(j.cdir + c);
+            slice_issue(j, d.off, (uint32_t)d.bytes, g + (uint32_t)c, bar, slots);
+        }
+
+    for (int c = 0; c < nch; ++c) {
+        const uint32_t gc = g + (uint32_t)c, par = (gc / NSLOT) & 1u;
+        const int slot = (int)(gc & (NSLOT - 1));
+        const uint8_t *chunk = slots + (size_t)slot * SLICE_SLOT;
+        const SliceTerm *terms = (const SliceTerm *)(chunk + SLICE_HEAD);
+        const bool ok = __all_sync(~0u, j.wait_limit > 0 ? mbar_poll(&bar[slot], par, j.wait_limit)
+                                                         : mbar_wait(&bar[slot], par));
+        const SliceChunk &d = *(const SliceChunk *)chunk;
+        const int nt = ok ? d.n_terms : 0;
+
+        // rows pass: one half term a warp
+        for (int task = tid >> 5; task < 2 * nt; task += nthr >> 5)
+                slice_task(chunk, terms[task < nt ? task : task - nt], task >= nt, planes, plane_bytes, ln);
+        if (__syncthreads_or(!ok)) {
+            if (tid == 0) {
+                atomicOr(j.status, (uint32_t)KSIM_FLAG_WAIT_TIMEOUT);
+                mbar_wait(&bar[slot], par);
+                if (c + 1 < nch) mbar_wait(&bar[slot ^ 1], ((gc + 1) / NSLOT) & 1u);
+            }
+            return false;
+        }
+
+        // values pass
+        if (warp_any) {
+            for (int t = 0; t < nt; ++t) {
+                const SliceTerm &T = terms[t];
+                const uint32_t fl = T.flags, xs = T.xs, tw = T.tab;
+#pragma unroll
+                for (int h = 0; h < (S == 8 ? 2 : 1); ++h) {
+                    constexpr int N = S == 1 ? 1 : 4;
+                    const uint8_t *pl = planes + (int)T.plane * plane_bytes + byte0 + 16 * h;
+                    const uint32_t xw = slice_plane<N>(pl), kw = slice_plane<N>(pl + plane_bytes);
+                    const uint32_t xm = xw & 0x7F7F7F7Fu, km = kw & 0x3F3F3F3Fu;
+                    const uint32_t base = fl & ST_BIG ? 0u : tw;
+                    uint32_t at[N];
+#pragma unroll
+                    for (int k = 0; k < N; ++k) at[k] = byte_of(xm, k) * xs + (byte_of(km, k) * 8u + base);
+                    if (fl & ST_WIDE) {
+                        const uint32_t cw = slice_plane<N>(pl + 2 * plane_bytes);
+                        const uint8_t *lut = chunk + 16 * (int)T.lut_off16;
+                        const uint32_t cs = (fl & ST_EVEN) ? 16u : 32u;
+#pragma unroll
+                        for (int k = 0; k < N; ++k) at[k] += (uint32_t)lut[byte_of(cw, k)] * cs;
+                    }
+                    // K's bit 1 has swapped the halves of the entry
+                    double a[N], b[N];
+                    if (fl & ST_BIG) {
+#pragma unroll
+                        for (int k = 0; k < N; ++k) {
+                            const uint8_t *p = kw & (0x40u << (8 * k)) ? j.image : j.image + 16 * (size_t)tw + at[k];
+                            const uint8_t *q = (const uint8_t *)((uintptr_t)p ^ 8u);
+                            a[k] = CG ? __ldcg((const double *)p) : __ldg((const double *)p);
+                            b[k] = CG ? __ldcg((const double *)q) : __ldg((const double *)q);
+                        }
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < N; ++k) {
+                            const uint32_t o = kw & (0x40u << (8 * k)) ? 0u : at[k];
+                            a[k] = *(const double *)(chunk + o);
+                            b[k] = *(const double *)(chunk + (o ^ 8u));
+                        }
+                    }
+                    // times i^(K1 + 2 (K2 ^ S)): the signs go to bit 63
+                    const uint32_t sI = xw ^ kw, sR = sI ^ (kw << 7);
+#pragma unroll
+                    for (int k = 0; k < N; ++k) {
+                        const int ra = (int)((sR << (24 - 8 * k)) & 0x80000000u);
+                        const int ib = (int)((sI << (24 - 8 * k)) & 0x80000000u);
+                        double &re = sre[4 * h + k], &im = sim[4 * h + k];
+                        re = dadd(re, __hiloint2double(__double2hiint(a[k]) ^ ra, __double2loint(a[k])));
+                        im = dadd(im, __hiloint2double(__double2hiint(b[k]) ^ ib, __double2loint(b[k])));
+                    }
+                }
+            }
+        }
+
+        if (d.end_of_graph) {
+            const int k = d.graph;
+            bool bit[S] = {};
+            if (warp_any) {
+#pragma unroll
+                for (int q = 0; q < S; ++q) {
+                    const double mag = dsqrt(dadd(dmul(sre[q], sre[q]), dmul(sim[q], sim[q])));
+                    sre[q] = 0.0;
+                    sim[q] = 0.0;
+                    const int64_t sh = sh_of(q);
+                    if (j.amp && ((act >> q) & 1u)) j.amp[sh * (int64_t)(j.n_out + 1) + k] = mag;
+                    if (k == 0) {
+                        prev[q] = mag;
+                    } else {
+                        const double u = j.rng_mode == KSIM_RNG_PHILOX
+                                             ? slice_philox(j.seed, (uint64_t)(j.shot_offset + sh), (uint32_t)(k - 1))
+                                             : slice_xorshift(rng[q]);
+                        bit[q] = slice_draw(u, mag, prev[q], ((act >> q) & 1u) ? flags : idle_flags);
+                        prev[q] = bit[q] ? mag : dsub(prev[q], mag);
+                    }
+                }
+            }
+            if (k == 0) {  // from graph 1 on, outputs not yet sampled are the trying bit
+                fill_rows(F, R, ~0u);
+            } else {
+                put_row(F + k - 1, bit);
+            }
+        }
+        const int64_t ahead_off = 16 * (int64_t)d.ahead_off16;
+        const uint32_t ahead_bytes = d.ahead_bytes;
+        __syncthreads();
+        if (tid == 0 && c + NSLOT < nch) slice_issue(j, ahead_off, ahead_bytes, gc + NSLOT, bar, slots);
+    }
+    g += (uint32_t)nch;
+
+    for (int i = 0; i < j.n_out && mine; ++i) {
+        const uint32_t x = *(const uint32_t *)(smem + (F + i) * SLICE_ROW + wcol) >> r;
+        const int64_t col = j.out_cols ? (int64_t)ldj<CG>(j.out_cols + i) : j.out_col0 + i;
+#pragma unroll
+        for (int k = 0; k < S; ++k)
+            if ((act >> k) & 1u)
+                j.out[sh_of(k) * j.out_stride + col] = (uint8_t)((x >> (S == 8 ? 8 * (k & 3) + 4 * (k >> 2) : 8 * k)) & 1u);
+    }
+    if (flags) atomicOr(j.status, flags);
+    return true;
+}
+
+}  // namespace ksim
