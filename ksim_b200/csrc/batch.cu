@@ -38,6 +38,7 @@
 #include "kernels.h"
 #include "runtime.h"
 #include "sample_tile.cuh"
+#include "slice_tile.cuh"
 
 namespace ksim {
 
@@ -48,7 +49,7 @@ struct BatchJobDev {
 };
 
 struct BatchItem {
-    int32_t job, pad;
+    int32_t job, shots;  // shots: of the tile
     int64_t s0;
 };
 
@@ -79,7 +80,7 @@ constexpr int BATCH_PARAM_JOBS = 180;
 struct BatchParams {
     const BatchItem *items;
     int *counter;
-    int32_t n_items, slot_bytes;
+    int32_t n_items, slot_bytes;  // slot_bytes: of a sliced class, its ring's offset
     BatchJobDev jobs[BATCH_PARAM_JOBS];
     __device__ __forceinline__ const BatchJobDev &job(int i) const { return jobs[i]; }
 };
@@ -145,6 +146,34 @@ __global__ void KSIM_BATCH_BOUNDS(PATHS) k_batch_c(const __grid_constant__ PT P)
     pdl_wait();
 }
 
+// A class whose jobs all have sliced streams: the sliced body (one for every W
+// and term path), 256 threads, four shots a thread; a tile's width is its
+// item's.
+template <typename PT>
+__global__ void __launch_bounds__(256, 2) k_batch_s(const __grid_constant__ PT P)
+{
+    extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ int s_item;
+    uint8_t *ring = smem + P.slot_bytes;
+    uint64_t *bar = (uint64_t *)ring;
+    ring_init(bar);
+    pdl_launch_dependents();
+    uint32_t g = 0;
+    for (;;) {
+        if (threadIdx.x == 0) s_item = atomicAdd(P.counter, 1);
+        __syncthreads();
+        const int it = s_item;
+        __syncthreads();
+        if (it >= P.n_items) break;
+        const BatchItem w = P.items[it];
+        const SampleJob &j = P.job(w.job).j;
+        const int64_t end = w.s0 + w.shots < j.B ? w.s0 + w.shots : j.B;
+        if (!slice_tile<4>(j, w.s0, end, w.shots, smem, slice_rows_bytes(j.s_rows, w.shots), bar, ring + BAR_BYTES, g))
+            break;
+    }
+    pdl_wait();
+}
+
 // The class with W in 5..16 (rare): the general body per W.
 template <typename PT>
 __global__ void __maxnreg__(255) k_batch_wide(const __grid_constant__ PT P)
@@ -181,8 +210,9 @@ __global__ void __maxnreg__(255) k_batch_wide(const __grid_constant__ PT P)
 
 // The kernel of class `cls` for job-table type PT.
 template <typename PT>
-const void *batch_kernel(int cls)
+const void *batch_kernel(int cls, bool sliced)
 {
+    if (sliced) return (const void *)k_batch_s<PT>;
 #define KSIM_BK(WW)                                                                  \
     case 3 * (WW - 1): return (const void *)k_batch_c<PT, WW, PATHS_NARROW>;         \
     case 3 * (WW - 1) + 1: return (const void *)k_batch_c<PT, WW, PATHS_NARROW_HYBRID>; \
@@ -205,9 +235,11 @@ namespace {
 // One class of a batch: launch shape and items.
 struct BatchClass {
     int threads = 128, slot = 14336, max_w = 1;
+    int ring_off = 0;       // of a sliced class: its CTAs' rows and planes
     size_t smem = 0;
     BatchItem *d_items = nullptr;
     int n_items = 0, grid = 0;
+    bool sliced = true;     // every job has a sliced stream
     bool high = false;      // hybrid, general and wide classes: launched before the 32-bit ones
     double head_cost = 0;   // cost of its costliest item
     std::unique_ptr<BatchParams> p;  // the job table by value (<= BATCH_PARAM_JOBS jobs)
@@ -255,10 +287,10 @@ static cudaError_t batch_launch_class(ksim_batch *b, int c, cudaStream_t st, boo
     lc.numAttrs = follow ? 1 : 0;
     if (k.p) {
         void *args[] = {(void *)k.p.get()};
-        return cudaLaunchKernelExC(&lc, batch_kernel<BatchParams>(c), args);
+        return cudaLaunchKernelExC(&lc, batch_kernel<BatchParams>(c, k.sliced), args);
     }
     void *args[] = {(void *)&k.pg};
-    return cudaLaunchKernelExC(&lc, batch_kernel<BatchParamsG>(c), args);
+    return cudaLaunchKernelExC(&lc, batch_kernel<BatchParamsG>(c, k.sliced), args);
 }
 
 static ksim_status batch_enqueue(ksim_batch *b, cudaStream_t st)
@@ -339,15 +371,29 @@ ksim_status ksim_batch_create(const ksim_batch_job *jobs, int32_t n_jobs, const 
             return fail(KSIM_ERR_INVALID_ARGUMENT, "job " + std::to_string(i) + ": a term record (" +
                                                        std::to_string(c->img.max_term_bytes) +
                                                        " bytes) exceeds slot_bytes");
+        k.sliced = k.sliced && c->cfg.sliced;
         if (need > k.slot) k.slot = (int)std::min<int64_t>(need, 1 << 30);
         k.max_w = std::max(k.max_w, c->img.W);
     }
     for (int c = 0; c < BATCH_CLASSES; ++c)
-        if (batch_smem_bytes(b->cls[c].slot, b->cls[c].max_w, b->cls[c].threads) > 227 * 1024)
+        if (!b->cls[c].sliced && batch_smem_bytes(b->cls[c].slot, b->cls[c].max_w, b->cls[c].threads) > 227 * 1024)
             return fail(KSIM_ERR_UNSUPPORTED, "a term record needs a staging slot of " +
                                                   std::to_string(b->cls[c].slot) + " bytes, beyond shared memory");
     b->device = device;
     DeviceGuard g(device);
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    // a sliced tile is as wide as the batch allows: 1,024 shots cost least a
+    // shot (one of 512 costs about 0.7 of it, of 256 about 0.55), but an item
+    // longer than a few percent of the whole batch's time would be its tail
+    double batch_time = 0;  // in terms of a 1,024-shot tile, per CTA slot
+    for (int i = 0; i < n_jobs; ++i)
+        batch_time += (double)jobs[i].comp->img.n_terms * ((double)((jobs[i].B + 1023) / 1024)) / (2.0 * std::max(sms, 1));
+    auto slice_shots = [&](const ksim_component *c) {
+        const double t = (double)c->img.n_terms;
+        const int most = b->threads <= 64 ? 512 : 1024;
+        return std::min(most, t <= 0.25 * batch_time ? 1024 : t <= 0.5 * batch_time ? 512 : 256);
+    };
     std::vector<BatchItem> items[BATCH_CLASSES];
     std::vector<double> cost[BATCH_CLASSES];
     for (int i = 0; i < n_jobs; ++i) {
@@ -359,6 +405,7 @@ ksim_status ksim_batch_create(const ksim_batch_job *jobs, int32_t n_jobs, const 
         cfg.threads = k.threads;
         cfg.staged = 1;
         cfg.slot_bytes = k.slot;
+        cfg.sliced = k.sliced ? 1 : 0;
         BatchJobDev d = {};
         ksim_status st = component_job(c, cfg, d.j);
         if (st != KSIM_OK) return st;
@@ -381,13 +428,16 @@ ksim_status ksim_batch_create(const ksim_batch_job *jobs, int32_t n_jobs, const 
         if (c->img.n_out == 0 || jb.B == 0) continue;
         double bytes = 0;
         for (const GraphDir &gd : c->img.gdir) bytes += (double)gd.stream_bytes + 64.0;
-        const int64_t tile = (int64_t)k.threads * shots_per_thread(d.W);
+        const int64_t tile = k.sliced ? slice_shots(c) : (int64_t)k.threads * shots_per_thread(d.W);
+        if (k.sliced) k.ring_off = std::max(k.ring_off, slice_ring_off(c->slice_rows, c->slice_planes, (int)tile));
         for (int64_t s0 = 0; s0 < jb.B; s0 += tile) {
             BatchItem it = {};
             it.job = i;
+            it.shots = (int32_t)tile;
             it.s0 = s0;
             items[cl].push_back(it);
-            cost[cl].push_back(bytes * (double)std::min<int64_t>(tile, jb.B - s0));
+            cost[cl].push_back(k.sliced ? (double)c->img.n_terms * (tile >= 1024 ? 1.0 : tile >= 512 ? 0.7 : 0.55)
+                                        : bytes * (double)std::min<int64_t>(tile, jb.B - s0));
         }
     }
     cudaError_t e = cudaMalloc(&b->d_jobs, sizeof(BatchJobDev) * b->host_jobs.size());
@@ -399,13 +449,13 @@ ksim_status ksim_batch_create(const ksim_batch_job *jobs, int32_t n_jobs, const 
         ksim_batch_destroy(b.release());
         return cuda_fail(e, "batch upload");
     }
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const bool by_value = b->host_jobs.size() <= (size_t)BATCH_PARAM_JOBS;
     for (int c = 0; c < BATCH_CLASSES; ++c) {
         BatchClass &k = b->cls[c];
         if (items[c].empty()) continue;
-        k.smem = batch_smem_bytes(k.slot, k.max_w, k.threads);
+        if (k.sliced) k.threads = 256;
+        k.smem = k.sliced ? (size_t)k.ring_off + BAR_BYTES + NSLOT * SLICE_SLOT
+                          : batch_smem_bytes(k.slot, k.max_w, k.threads);
         std::vector<int> order(items[c].size());
         std::iota(order.begin(), order.end(), 0);
         std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[c][x] > cost[c][y]; });
@@ -423,19 +473,20 @@ ksim_status ksim_batch_create(const ksim_batch_job *jobs, int32_t n_jobs, const 
             k.p->items = k.d_items;
             k.p->counter = b->d_counter + c;
             k.p->n_items = k.n_items;
-            k.p->slot_bytes = k.slot;
+            k.p->slot_bytes = k.sliced ? k.ring_off : k.slot;
             std::copy(b->host_jobs.begin(), b->host_jobs.end(), k.p->jobs);
         } else {
             k.pg.items = k.d_items;
             k.pg.counter = b->d_counter + c;
             k.pg.n_items = k.n_items;
-            k.pg.slot_bytes = k.slot;
+            k.pg.slot_bytes = k.sliced ? k.ring_off : k.slot;
             k.pg.gjobs = b->d_jobs;
         }
         int active = 0;
         if (e == cudaSuccess) {
-            const void *fn = by_value ? batch_kernel<BatchParams>(c) : batch_kernel<BatchParamsG>(c);
-            e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem);
+            const void *fn = by_value ? batch_kernel<BatchParams>(c, k.sliced) : batch_kernel<BatchParamsG>(c, k.sliced);
+            e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     k.sliced ? SLICE_SMEM_MAX : (int)k.smem);
             if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&active, fn, k.threads, k.smem);
         }
         if (e != cudaSuccess) {

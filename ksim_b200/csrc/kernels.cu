@@ -135,7 +135,8 @@ cudaError_t launch_slice_as(const SampleJob &j, int shots, int threads, int tile
     const int64_t blocks = (j.B + tile - 1) / tile;
     if (blocks > 0x7FFFFFFF) return cudaErrorInvalidConfiguration;
     const int smem = slice_smem_bytes(j.s_rows, j.s_planes, shots);
-    cudaError_t e = cudaFuncSetAttribute(k_slice<S, THREADS, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(k_slice<S, THREADS, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         SLICE_SMEM_MAX);
     if (e != cudaSuccess) return e;
     k_slice<S, THREADS, CTAS><<<(unsigned)blocks, threads, smem, st>>>(j, shots, tile);
     return cudaGetLastError();

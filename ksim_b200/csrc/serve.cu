@@ -7,7 +7,7 @@
 // the next, so the tiles of every request admitted so far are handed out in
 // arrival order while earlier requests are still running on other CTAs.  The
 // CTA copies the job's descriptor into shared memory with L2-only loads and
-// runs the sampling tile (sample_tile.cuh, L2-coherent loads, one staging
+// runs the sliced sampling tile (slice_tile.cuh, L2-coherent loads, one staging
 // ring per CTA for its whole life).  The CTA that finishes a job's last tile
 // decrements the request's job count; the one that finishes the request
 // writes the request's sequence number into a host-mapped flag after a
@@ -30,9 +30,9 @@
 //   3. polls the completion flags, copies finished outputs (and the request's
 //      status word) to the caller's buffer on a second copy stream, and frees
 //      the request's resources once that copy is done.
-// Programs with parameter vectors wider than 256 bits (W > 4) are not in the
-// loop kernel's instantiations; their requests run as plain launches on a
-// side stream, admitted and completed through the same queue.
+// Programs with a component that has no sliced stream (more than 254
+// parameters, terms without a range proof) run as plain launches on a side
+// stream, admitted and completed through the same queue.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -51,15 +51,16 @@
 #include "runtime.h"
 #include "sample_tile.cuh"
 #include "serve_sched.h"
+#include "slice_tile.cuh"
 
 namespace ksim {
 
 struct ServeJob {
     SampleJob j;
-    int32_t W, n_tiles;
+    int32_t shots, n_tiles;  // shots of a tile
     int32_t next_tile;  // tiles handed out (atomic)
     int32_t remaining;  // tiles not finished (atomic)
-    int32_t req_slot, paths;  // paths: the component's term paths (LaunchCfg::paths)
+    int32_t req_slot, pad0;
     int64_t pad1;
 };
 static_assert(sizeof(SampleJob) % 16 == 0, "SampleJob is copied in 16-byte words");
@@ -97,27 +98,20 @@ __device__ __forceinline__ T vload(const T *p)
     return *(const volatile T *)p;
 }
 
-// One tile of a job with the body compiled for the job's W and term paths.
-// The loop inlines the bodies that carry most requests (all-32-bit W = 1
-// and 2, 32-bit and hybrid W = 2) and calls the others out of line (a call
-// costs the body about a tenth of its speed; inlining every body would
-// bloat the loop).  Job data comes through L2-only loads (CG): buffers are
-// reused across requests within one kernel lifetime.
-template <int W, int PATHS>
-__device__ __noinline__ bool serve_tile(const SampleJob &j, int64_t s0, uint64_t *bar, uint8_t *slots, uint32_t &g,
-                                        uint8_t *scratch)
-{
-    return sample_tile<W, true, true, shots_per_thread(W), PATHS>(j, s0, bar, slots, g, scratch);
-}
+// Shared memory of the loop's CTAs: any sliced job's parameter rows and
+// planes, then one ring for the CTA's whole life.
+constexpr int SERVE_THREADS = 256;
+constexpr int SERVE_SHOTS = 1024;  // widest tile
+constexpr int SERVE_RING = slice_ring_off(SLICE_MAX_ROWS, SLICE_MAX_PLANES, SERVE_SHOTS);
+constexpr int SERVE_SMEM = slice_smem_bytes(SLICE_MAX_ROWS, SLICE_MAX_PLANES, SERVE_SHOTS);
 
-__global__ void __launch_bounds__(256, KSIM_SAMPLE_MIN_CTAS) k_serve(ServeJob *jobs, ServeReqDev *reqs, const unsigned long long *ring,
+__global__ void __launch_bounds__(SERVE_THREADS, 2) k_serve(ServeJob *jobs, ServeReqDev *reqs, const unsigned long long *ring,
                                                int ring_cap, ServeCtl *ctl, uint32_t *done_flags, long long idle_ns)
 {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ __align__(16) SampleJob s_job;
-    __shared__ int s_slot, s_tile, s_W, s_paths;
-    uint64_t *bar = (uint64_t *)smem;
-    uint8_t *slots = smem + BAR_BYTES;
+    __shared__ int s_slot, s_tile, s_shots;
+    uint64_t *bar = (uint64_t *)(smem + SERVE_RING);
     ring_init(bar);
     uint32_t g = 0;
     const long long t_start = global_ns();
@@ -141,8 +135,7 @@ __global__ void __launch_bounds__(256, KSIM_SAMPLE_MIN_CTAS) k_serve(ServeJob *j
             if (slot >= 0) {
                 backoff = 64;
                 *(volatile long long *)&ctl->last_claim_ns = global_ns();
-                s_W = vload(&jobs[slot].W);
-                s_paths = vload(&jobs[slot].paths);
+                s_shots = vload(&jobs[slot].shots);
             } else {
                 const long long now = global_ns();
                 const long long last = vload(&ctl->last_claim_ns);
@@ -168,32 +161,11 @@ __global__ void __launch_bounds__(256, KSIM_SAMPLE_MIN_CTAS) k_serve(ServeJob *j
         }
         __syncthreads();
         if (slot >= 0) {
-            constexpr int S = shots_per_thread(4);  // every loop job has W <= 4
-            const int64_t s0 = (int64_t)s_tile * blockDim.x * S;
-            uint8_t *scratch = slots + (size_t)NSLOT * s_job.slot_bytes;
-            bool ok;
-            const int paths = s_paths;
-#define KSIM_SERVE_W(WW)                                                                                \
-    case WW:                                                                                            \
-        ok = paths == PATHS_NARROW ? serve_tile<WW, PATHS_NARROW>(s_job, s0, bar, slots, g, scratch)    \
-             : paths == PATHS_NARROW_HYBRID                                                             \
-                 ? serve_tile<WW, PATHS_NARROW_HYBRID>(s_job, s0, bar, slots, g, scratch)              \
-                 : serve_tile<WW, PATHS_ALL>(s_job, s0, bar, slots, g, scratch);                       \
-        break;
-            // the common bodies inline, the rest out of line
-            if (s_W == 1 && paths == PATHS_NARROW)
-                ok = sample_tile<1, true, true, shots_per_thread(1), PATHS_NARROW>(s_job, s0, bar, slots, g, scratch);
-            else if (s_W == 2 && paths == PATHS_NARROW)
-                ok = sample_tile<2, true, true, shots_per_thread(2), PATHS_NARROW>(s_job, s0, bar, slots, g, scratch);
-            else if (s_W == 2 && paths == PATHS_NARROW_HYBRID)
-                ok = sample_tile<2, true, true, shots_per_thread(2), PATHS_NARROW_HYBRID>(s_job, s0, bar, slots, g, scratch);
-            else {
-            switch (s_W) {
-            KSIM_SERVE_W(1) KSIM_SERVE_W(2) KSIM_SERVE_W(3)
-            default: KSIM_SERVE_W(4)
-            }
-            }
-#undef KSIM_SERVE_W
+            const int shots = s_shots;
+            const int64_t s0 = (int64_t)s_tile * shots;
+            const bool ok = slice_tile<4, true>(s_job, s0, s0 + shots < s_job.B ? s0 + shots : s_job.B, shots, smem,
+                                                slice_rows_bytes(s_job.s_rows, shots), bar,
+                                                smem + SERVE_RING + BAR_BYTES, g);
             __threadfence();  // this thread's outputs before the counters below
             __syncthreads();
             if (threadIdx.x == 0) {
@@ -253,7 +225,6 @@ struct ksim_server {
     ksim_server_config cfg = {};
     LaunchCfg lcfg;
     int grid = 0;
-    size_t smem = 0;
 
     uint8_t *d_arena = nullptr;
     Arena arena;
@@ -318,13 +289,6 @@ void release(ksim_server *s, ServeRequest *r)
     r->ev = nullptr;
 }
 
-int words_of(const ksim_program *p)
-{
-    int w = 1;
-    for (const ProgramPart &part : p->parts) w = std::max(w, part.comp->img.W);
-    return w;
-}
-
 // Admit and publish one request (caller holds mu; resources were checked).
 ksim_status admit(ksim_server *s, ServeRequest *r)
 {
@@ -357,8 +321,11 @@ ksim_status admit(ksim_server *s, ServeRequest *r)
         r->state = R_RUNNING;
         return KSIM_OK;
     }
-    // job descriptors
-    const int64_t tile = (int64_t)s->lcfg.threads * shots_per_thread(4);
+    // job descriptors.  Few shots take narrow tiles (a tile of 512 shots ends
+    // in about 0.7 of the time of one of 1,024, 256 in 0.55), many the wide
+    // ones, which cost least a shot
+    const int64_t by_shots = r->B <= 128 ? 128 : r->B <= 1024 ? 256 : r->B <= 8192 ? 512 : SERVE_SHOTS;
+    const int64_t tile = s->cfg.threads > 0 ? std::min<int64_t>(by_shots, 4 * s->cfg.threads) : by_shots;
     const int64_t tiles = (r->B + tile - 1) / tile;
     std::vector<int> new_jobs;
     for (size_t k = 0; k < p->parts.size(); ++k) {
@@ -385,8 +352,7 @@ ksim_status admit(ksim_server *s, ServeRequest *r)
         J.j.shot_offset = 0;
         J.j.seed = r->seed + 0x9E37ull * (uint64_t)k;
         J.j.status = &s->d_reqs[r->slot].flags;
-        J.W = c->img.W;
-        J.paths = c->cfg.paths;
+        J.shots = (int32_t)tile;
         J.n_tiles = (int32_t)tiles;
         J.next_tile = 0;
         J.remaining = (int32_t)tiles;
@@ -433,7 +399,7 @@ void ensure_loop(ksim_server *s)
     if (e == cudaSuccess) e = cudaStreamWaitEvent(s->s_loop, s->h2d_mark, 0);
     if (e == cudaSuccess) e = cudaMemsetAsync(&s->d_ctl->exiting, 0, sizeof(int32_t), s->s_loop);
     if (e == cudaSuccess) {
-        k_serve<<<s->grid, s->lcfg.threads, s->smem, s->s_loop>>>(s->d_jobs, s->d_reqs, s->d_ring, s->ring_cap,
+        k_serve<<<s->grid, SERVE_THREADS, SERVE_SMEM, s->s_loop>>>(s->d_jobs, s->d_reqs, s->d_ring, s->ring_cap,
                                                                    s->d_ctl, s->d_done,
                                                                    (long long)s->cfg.idle_us * 1000ll);
         e = cudaGetLastError();
@@ -590,6 +556,7 @@ ksim_status ksim_server_create(const ksim_server_config *cfg_in, ksim_server **o
     if (cfg.arena_bytes <= 0) cfg.arena_bytes = (int64_t)1 << 30;
     if (cfg.max_requests <= 0) cfg.max_requests = 1024;
     if (cfg.max_jobs <= 0) cfg.max_jobs = 4096;
+    const bool threads_given = cfg.threads > 0;
     if (cfg.threads <= 0) cfg.threads = 128;
     if (cfg.slot_bytes <= 0) cfg.slot_bytes = 16384;
     if (cfg.idle_us <= 0) cfg.idle_us = 2000;
@@ -601,9 +568,9 @@ ksim_status ksim_server_create(const ksim_server_config *cfg_in, ksim_server **o
     std::unique_ptr<ksim_server> s(new ksim_server());
     s->device = cfg.device;
     s->cfg = cfg;
-    s->lcfg.threads = cfg.threads;
-    s->lcfg.staged = 1;
-    s->lcfg.slot_bytes = cfg.slot_bytes;
+    // the caller's threads set the widest tile (a power of two)
+    s->cfg.threads = threads_given ? (cfg.threads >= 256 ? 256 : cfg.threads >= 128 ? 128 : cfg.threads >= 64 ? 64 : 32) : 0;
+    s->lcfg.sliced = 1;
     s->ring_cap = cfg.max_jobs;
     DeviceGuard g(cfg.device);
     if (!g.ok) return fail(KSIM_ERR_INVALID_ARGUMENT, "cannot select device " + std::to_string(cfg.device));
@@ -644,11 +611,10 @@ ksim_status ksim_server_create(const ksim_server_config *cfg_in, ksim_server **o
         if ((e = cudaStreamCreateWithFlags(st, cudaStreamNonBlocking)) != cudaSuccess) return bail(e, "streams");
     if ((e = cudaEventCreateWithFlags(&s->loop_done, cudaEventDisableTiming)) != cudaSuccess) return bail(e, "events");
     if ((e = cudaEventCreateWithFlags(&s->h2d_mark, cudaEventDisableTiming)) != cudaSuccess) return bail(e, "events");
-    s->smem = sample_smem_bytes(cfg.slot_bytes, true, 4, cfg.threads);
-    if ((e = cudaFuncSetAttribute(k_serve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s->smem)) != cudaSuccess)
+    if ((e = cudaFuncSetAttribute(k_serve, cudaFuncAttributeMaxDynamicSharedMemorySize, SERVE_SMEM)) != cudaSuccess)
         return bail(e, "loop kernel attributes");
     int active = 0, sms = 0;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&active, k_serve, cfg.threads, s->smem)) != cudaSuccess)
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&active, k_serve, SERVE_THREADS, SERVE_SMEM)) != cudaSuccess)
         return bail(e, "loop kernel occupancy");
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg.device);
     const int per_sm = cfg.ctas_per_sm > 0 ? std::min(cfg.ctas_per_sm, std::max(active, 1)) : std::max(active, 1);
@@ -686,15 +652,11 @@ ksim_status ksim_server_submit(ksim_server *s, ksim_program *p, const uint8_t *f
     r->out_bytes = B * p->n_outputs;
     r->seed = seed;
     r->rng_mode = rng_mode;
-    r->loop = words_of(p) <= 4;
+    // the loop runs sliced streams; a program with a component that has none
+    // runs as plain launches
+    for (const ProgramPart &part : p->parts) r->loop = r->loop && part.comp->cfg.sliced;
     for (const ProgramPart &part : p->parts) r->n_jobs += part.comp->img.n_out > 0 ? 1 : 0;
     r->t_submit = Clock::now();
-    // every component needs its chunk directory for the loop's slot size
-    if (r->loop)
-        for (const ProgramPart &part : p->parts) {
-            if (part.comp->img.max_term_bytes > s->lcfg.slot_bytes)
-                r->loop = false;  // a term larger than the loop's slot: plain launch
-        }
     std::lock_guard<std::mutex> lk(s->mu);
     if (s->stopping) return fail(KSIM_ERR_INVALID_ARGUMENT, "server is shutting down");
     if (!s->fatal.empty()) return fail(KSIM_ERR_CUDA, s->fatal);

@@ -41,6 +41,12 @@ __host__ __device__ constexpr int slice_smem_bytes(int rows, int planes, int sho
     return slice_ring_off(rows, planes, shots) + BAR_BYTES + NSLOT * SLICE_SLOT;
 }
 
+// The most a sliced CTA takes (254 parameters, 2,048 shots): every sliced
+// kernel's dynamic shared-memory bound, whatever a launch asks for, so
+// launches from several threads do not lower it for one another.
+constexpr int SLICE_SMEM_MAX = slice_smem_bytes(SLICE_MAX_ROWS, SLICE_MAX_PLANES, 2048);
+static_assert(SLICE_SMEM_MAX <= 226 * 1024, "shared memory of a CTA");
+
 struct W2 {
     uint32_t a, b;
 };
@@ -319,11 +325,11 @@ __device__ __forceinline__ void slice_task(const uint8_t *chunk, const SliceTerm
 // of it relatively (normal t), so outside t (1 +- 2^-50) the quotient's
 // rounding cannot change the comparison.  Everything else (and NaN, zeros,
 // infinities beside infinities) divides.  flags: KSIM_FLAG_* raised.
-__device__ __noinline__ double slice_philox(uint64_t seed, uint64_t shot, uint32_t output)
+static __device__ __noinline__ double slice_philox(uint64_t seed, uint64_t shot, uint32_t output)
 {
     return philox_uniform(seed, shot, output);
 }
-__device__ __noinline__ uint32_t slice_draw_exact(double u, double mag, double prev)
+static __device__ __noinline__ uint32_t slice_draw_exact(double u, double mag, double prev)
 {
     const double ratio = __ddiv_rn(mag, prev);
     return (u < ratio ? 1u : 0u) | (!(prev > 0.0) ? (uint32_t)KSIM_FLAG_PREV_NONPOSITIVE << 8 : 0u) |
