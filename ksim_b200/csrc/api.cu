@@ -218,6 +218,8 @@ ksim_status ksim_component_create(const ksim_graph_desc *graphs, int32_t n_graph
         if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpy(sliced stream)");
         c->d_slice_dir = (const ChunkDir *)(c->d_slices + at);
         c->slice_chunks = (int)sl.chunks.size();
+        c->slice_first.assign((size_t)n_graphs + 1, c->slice_chunks);
+        for (int i = c->slice_chunks - 1; i >= 0; --i) c->slice_first[(size_t)sl.chunks[i].graph] = i;
         c->slice_rows = sl.rows;
         c->slice_planes = sl.max_planes;
         c->cfg.sliced = 1;
@@ -429,6 +431,32 @@ static ksim_status eval_common(ksim_component *c, int32_t graph, const uint8_t *
     if (P > 0) {
         e = cudaMemcpyAsync(c->ws_f.p, params, (size_t)(B * P), cudaMemcpyHostToDevice, c->stream);
         if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync(params)");
+    }
+    if (c->cfg.sliced && mode != EVAL_TERMS) {
+        // the sampling kernel's two passes on this graph's chunks: the rows are
+        // the parameter vectors (parameters past the component's are in no
+        // mask)
+        LaunchCfg cfg = c->cfg;
+        cfg.slice_threads = 0;
+        SampleJob s = {};
+        s.image = c->d_slices;
+        s.cdir = c->d_slice_dir + c->slice_first[(size_t)graph];
+        s.n_chunks = c->slice_first[(size_t)graph + 1] - c->slice_first[(size_t)graph];
+        s.F = (int32_t)std::min<int64_t>(P, c->slice_rows);
+        s.s_rows = c->slice_rows;
+        s.s_planes = c->slice_planes;
+        s.f = (const uint8_t *)c->ws_f.p;
+        s.f_stride = P;
+        s.amp = (double *)c->ws_aux.p;
+        s.B = B;
+        s.status = c->d_status;
+        e = launch_eval_sliced(s, mode, cfg, c->stream);
+        if (e != cudaSuccess) return cuda_fail(e, "eval kernel launch");
+        e = cudaMemcpyAsync(out, c->ws_aux.p, out_bytes, cudaMemcpyDeviceToHost, c->stream);
+        if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync(eval out)");
+        e = cudaStreamSynchronize(c->stream);
+        if (e != cudaSuccess) return cuda_fail(e, "eval");
+        return KSIM_OK;
     }
     EvalJob j = {};
     j.image = c->d_image;

@@ -39,7 +39,8 @@ __global__ void KSIM_SAMPLE_BOUNDS(PATHS) k_sample(const SampleJob j)
 
 // The sliced sampler: one CTA per `tile` shots (tile <= shots, the width of
 // the CTA's bit rows).  S shots a thread; THREADS and CTAS bound the registers.
-template <int S, int THREADS, int CTAS>
+// EVAL: as slice_tile's.
+template <int S, int THREADS, int CTAS, int EVAL>
 __global__ void __launch_bounds__(THREADS, CTAS) k_slice(const SampleJob j, const int shots, const int tile)
 {
     extern __shared__ __align__(128) uint8_t smem[];
@@ -48,7 +49,7 @@ __global__ void __launch_bounds__(THREADS, CTAS) k_slice(const SampleJob j, cons
     ring_init(bar);
     uint32_t g = 0;
     const int64_t s0 = (int64_t)blockIdx.x * tile;
-    slice_tile<S>(j, s0, s0 + tile < j.B ? s0 + tile : j.B, shots, smem, slice_rows_bytes(j.s_rows, shots), bar,
+    slice_tile<S, false, EVAL>(j, s0, s0 + tile < j.B ? s0 + tile : j.B, shots, smem, slice_rows_bytes(j.s_rows, shots), bar,
                   ring + BAR_BYTES, g);
 }
 
@@ -129,16 +130,16 @@ cudaError_t launch_sample_w(const SampleJob &j, const LaunchCfg &cfg, cudaStream
     return cudaGetLastError();
 }
 
-template <int S, int THREADS, int CTAS>
+template <int S, int THREADS, int CTAS, int EVAL>
 cudaError_t launch_slice_as(const SampleJob &j, int shots, int threads, int tile, cudaStream_t st)
 {
     const int64_t blocks = (j.B + tile - 1) / tile;
     if (blocks > 0x7FFFFFFF) return cudaErrorInvalidConfiguration;
     const int smem = slice_smem_bytes(j.s_rows, j.s_planes, shots);
-    cudaError_t e = cudaFuncSetAttribute(k_slice<S, THREADS, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(k_slice<S, THREADS, CTAS, EVAL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          SLICE_SMEM_MAX);
     if (e != cudaSuccess) return e;
-    k_slice<S, THREADS, CTAS><<<(unsigned)blocks, threads, smem, st>>>(j, shots, tile);
+    k_slice<S, THREADS, CTAS, EVAL><<<(unsigned)blocks, threads, smem, st>>>(j, shots, tile);
     return cudaGetLastError();
 }
 
@@ -153,26 +154,27 @@ cudaError_t launch_slice_as(const SampleJob &j, int shots, int threads, int tile
 //   500,000                    1.84  1.43 1.08 0.92
 // and alike on the 16-output t = 20 one: the widest tile costs least per shot,
 // but a narrower one that still fits one wave ends sooner.
+template <int EVAL = -1>
 cudaError_t launch_slice(const SampleJob &j, const LaunchCfg &cfg, cudaStream_t st)
 {
     if (cfg.slice_threads > 0) {  // threads chosen by the caller: four shots each
         const int t = cfg.slice_threads >= 256 ? 256 : cfg.slice_threads >= 128 ? 128 : cfg.slice_threads >= 64 ? 64 : 32;
-        return launch_slice_as<4, 256, 2>(j, 4 * t, t, 4 * t, st);
+        return launch_slice_as<4, 256, 2, EVAL>(j, 4 * t, t, 4 * t, st);
     }
     const int64_t sms = cfg.sms;
     if (j.B <= sms * 512) {
         const int shots = j.B <= sms * 128 ? 128 : j.B <= sms * 256 ? 256 : 512;
-        return launch_slice_as<1, 512, 1>(j, shots, 512, shots, st);
+        return launch_slice_as<1, 512, 1, EVAL>(j, shots, 512, shots, st);
     }
-    if (j.B <= sms * 1024) return launch_slice_as<4, 512, 1>(j, 1024, 512, 1024, st);
+    if (j.B <= sms * 1024) return launch_slice_as<4, 512, 1, EVAL>(j, 1024, 512, 1024, st);
     const bool wide = j.B > 2 * sms * 1024;
     const int shots = wide ? 2048 : 1024;
     // equal tiles: a last wave that is nearly empty costs as much as a full one
     const int64_t waves = (j.B + 2 * sms * shots - 1) / (2 * sms * shots);
     const int64_t want = (j.B + waves * 2 * sms - 1) / (waves * 2 * sms);
     const int tile = (int)((want + 63) / 64 * 64);
-    if (wide) return launch_slice_as<8, 256, 2>(j, shots, 256, tile, st);
-    return launch_slice_as<4, 256, 2>(j, shots, 256, tile, st);
+    if (wide) return launch_slice_as<8, 256, 2, EVAL>(j, shots, 256, tile, st);
+    return launch_slice_as<4, 256, 2, EVAL>(j, shots, 256, tile, st);
 }
 
 template <int W>
@@ -259,6 +261,12 @@ cudaError_t launch_sample(const SampleJob &job, int W, const LaunchCfg &cfg, cud
     case 16: return launch_sample_w<16>(job, cfg, st);
     default: return cudaErrorInvalidValue;
     }
+}
+
+cudaError_t launch_eval_sliced(const SampleJob &job, int mode, const LaunchCfg &cfg, cudaStream_t st)
+{
+    if (job.B <= 0) return cudaSuccess;
+    return mode == EVAL_ABS ? launch_slice<EVAL_ABS>(job, cfg, st) : launch_slice<EVAL_COMPLEX>(job, cfg, st);
 }
 
 cudaError_t launch_eval(const EvalJob &job, int W, cudaStream_t st)

@@ -52,6 +52,7 @@ struct ksim_component {
     uint8_t *d_slices = nullptr;
     const ksim::ChunkDir *d_slice_dir = nullptr;
     int slice_chunks = 0, slice_rows = 0, slice_planes = 0;
+    std::vector<int> slice_first;  // per graph: its first chunk (and the end)
     uint32_t *d_status = nullptr;
     cudaStream_t stream = nullptr;
     ksim::DevBuf ws_f, ws_out, ws_aux;

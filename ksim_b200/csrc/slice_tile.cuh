@@ -383,7 +383,9 @@ __device__ __forceinline__ void slice_issue(const SampleJob &j, int64_t off, uin
 // (shots / S threads; the others only share the rows pass).  smem: the CTA's shared
 // memory, parameter rows first, planes at planes_off.  Returns false after a
 // wait timeout (the CTA must then stop using the ring).
-template <int S, bool CG = false>
+// EVAL: instead of sampling, the job's chunks are one graph's and its rows are
+// whole parameter vectors; |A| (EVAL_ABS) or A (EVAL_COMPLEX) goes to j.amp.
+template <int S, bool CG = false, int EVAL = -1>
 __device__ __forceinline__ bool slice_tile(const SampleJob &j, const int64_t s0, const int64_t s_end, int shots,
                                            uint8_t *smem, int planes_off, uint64_t *bar, uint8_t *slots, uint32_t &g)
 {
@@ -575,7 +577,20 @@ __device__ __forceinline__ bool slice_tile(const SampleJob &j, const int64_t s0,
             }
         }
 
-        if (d.end_of_graph) {
+        if (EVAL >= 0) {
+            if (d.end_of_graph) {
+#pragma unroll
+                for (int q = 0; q < S; ++q) {
+                    if (!((act >> q) & 1u)) continue;
+                    if (EVAL == EVAL_ABS) {
+                        j.amp[sh_of(q)] = dsqrt(dadd(dmul(sre[q], sre[q]), dmul(sim[q], sim[q])));
+                    } else {
+                        j.amp[2 * sh_of(q)] = sre[q];
+                        j.amp[2 * sh_of(q) + 1] = sim[q];
+                    }
+                }
+            }
+        } else if (d.end_of_graph) {
             const int k = d.graph;
             bool bit[S] = {};
             if (warp_any) {
@@ -609,6 +624,7 @@ __device__ __forceinline__ bool slice_tile(const SampleJob &j, const int64_t s0,
         if (tid == 0 && c + NSLOT < nch) slice_issue(j, ahead_off, ahead_bytes, gc + NSLOT, bar, slots);
     }
     g += (uint32_t)nch;
+    if (EVAL >= 0) return true;
 
     for (int i = 0; i < j.n_out && mine; ++i) {
         const uint32_t x = *(const uint32_t *)(smem + (F + i) * SLICE_ROW + wcol) >> r;
