@@ -588,6 +588,7 @@ ksim_status ksim_program_create(ksim_component *const *comps, int32_t n_comps, c
     }
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
+    p->sms = std::max(sms, 1);
     p->wave_shots = (int64_t)std::max(sms, 1) * 5 * 256;  // five CTAs of 256 shots per SM
     cudaError_t e = cudaMallocHost(&p->h_status, sizeof(uint32_t) * std::max<size_t>(p->parts.size(), 1));
     if (e != cudaSuccess) {
@@ -650,9 +651,11 @@ ksim_status ksim_program_job(const ksim_program *p, int32_t k, const uint8_t *d_
 }
 int32_t ksim_program_min_f_cols(const ksim_program *p) { return p ? p->min_f_cols : -1; }
 
-ksim_status ksim_program_sample_device(ksim_program *p, const uint8_t *d_f_params, int64_t B, int64_t n_f_cols,
+// call_shots: shots of the whole call when this is one of several launches
+// that run together (0: of this launch alone).
+static ksim_status program_launch(ksim_program *p, const uint8_t *d_f_params, int64_t B, int64_t n_f_cols,
                                        int64_t shot_offset, uint64_t seed, int32_t rng_mode, uint8_t *d_out,
-                                       void *stream)
+                                  void *stream, int64_t call_shots)
 {
     if (!p) return fail(KSIM_ERR_INVALID_ARGUMENT, "program is NULL");
     if (B < 0 || shot_offset < 0) return fail(KSIM_ERR_INVALID_ARGUMENT, "B and shot_offset must be >= 0");
@@ -672,6 +675,7 @@ ksim_status ksim_program_sample_device(ksim_program *p, const uint8_t *d_f_param
             std::lock_guard<std::mutex> lk(c->mu);
             cfg = c->cfg;
         }
+        cfg.call_shots = call_shots;
         SampleJob j = {};
         ksim_status st = component_job(c, cfg, j);
         if (st != KSIM_OK) return st;
@@ -689,6 +693,14 @@ ksim_status ksim_program_sample_device(ksim_program *p, const uint8_t *d_f_param
         if (e != cudaSuccess) return cuda_fail(e, "sample kernel launch");
     }
     return KSIM_OK;
+}
+
+
+ksim_status ksim_program_sample_device(ksim_program *p, const uint8_t *d_f_params, int64_t B, int64_t n_f_cols,
+                                       int64_t shot_offset, uint64_t seed, int32_t rng_mode, uint8_t *d_out,
+                                       void *stream)
+{
+    return program_launch(p, d_f_params, B, n_f_cols, shot_offset, seed, rng_mode, d_out, stream, 0);
 }
 
 }  // extern "C"
@@ -731,7 +743,18 @@ ksim_status program_sample_host(ksim_program *p, const uint8_t *f, int64_t B, in
     uint8_t *d_in = packed ? (uint8_t *)p->ws_fp.p : d_f;       // where the host rows land
     uint8_t *d_back = packed ? (uint8_t *)p->ws_op.p : d_out;   // what goes back
 
-    const std::vector<int64_t> bounds = host_chunk_bounds(B, (noise ? 0 : f_row) + o_row);
+    // sliced kernels that outlast the copies: chunks that fill the SMs; else
+    // (copies dominate, or other kernels) the ramped plan
+    bool sliced = true;
+    double kernel_us = 0;  // of one tile per SM: 0.9 us a term, 1.2 a graph
+    for (const ProgramPart &part : p->parts) {
+        sliced = sliced && (part.comp->cfg.sliced || part.comp->img.n_out == 0);
+        kernel_us += 0.9 * (double)part.comp->img.n_terms + 1.2 * (double)part.comp->img.n_graphs;
+    }
+    const double copy_us = (double)B * (double)((noise ? 0 : f_row) + o_row) / 5e4;  // at 50 GB/s
+    const bool fill = sliced && 4 * kernel_us > copy_us;
+    const std::vector<int64_t> bounds = fill ? slice_chunk_bounds(B, p->sms)
+                                             : host_chunk_bounds(B, (noise ? 0 : f_row) + o_row);
     const int n_chunks = (int)bounds.size() - 1;
     const int lag = host_copy_lag(bounds, p->wave_shots, KSIM_HOST_STREAMS);
     std::vector<cudaEvent_t> &ev_in = p->ev_in, &ev_done = p->ev_done;
@@ -770,8 +793,8 @@ ksim_status program_sample_host(ksim_program *p, const uint8_t *f, int64_t B, in
         if (e == cudaSuccess && packed)
             e = launch_unpack_bits(d_in + c0 * f_row, n, f_row, n_f_cols, d_f + c0 * n_f_cols, cs);
         if (e != cudaSuccess) break;
-        st = ksim_program_sample_device(p, d_f + c0 * n_f_cols, n, n_f_cols, c0, seed, rng_mode, d_out + c0 * n_out,
-                                        cs);
+        st = program_launch(p, d_f + c0 * n_f_cols, n, n_f_cols, c0, seed, rng_mode, d_out + c0 * n_out, cs,
+                            n_chunks > 1 ? B : 0);
         if (st != KSIM_OK) break;
         if (packed) e = launch_pack_bits(d_out + c0 * n_out, n, n_out, o_row, d_back + c0 * o_row, cs);
         if (e == cudaSuccess) e = cudaEventRecord(ev_done[i], cs);

@@ -39,6 +39,19 @@ inline std::vector<int64_t> host_chunk_bounds(int64_t B, int64_t row_bytes)
     return b;
 }
 
+// Chunk boundaries of a host call whose kernels are the sliced ones: a chunk of
+// fewer shots than fill every SM once (sms x 512) takes about as long as a full
+// one, so the call is cut into such chunks, the last one taking up to a
+// quarter more.
+inline std::vector<int64_t> slice_chunk_bounds(int64_t B, int64_t sms)
+{
+    const int64_t u = sms * 512;
+    std::vector<int64_t> b = {0};
+    for (int64_t x = u; x + u / 4 < B; x += u) b.push_back(x);
+    b.push_back(B);
+    return b;
+}
+
 // How many chunks behind the sampling a call issues each chunk's output
 // copy: one wave of sampling CTAs (wave_shots) over the largest chunk,
 // between 1 and max_lag (the compute streams).  Into page-locked memory the

@@ -9,6 +9,8 @@
 // of kokkos_sim.cpp:157-185 (and the per-term numerator dump).
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "../../include/ksim_b200.h"
 #include "kernels.h"
 #include "sample_tile.cuh"
@@ -162,16 +164,20 @@ cudaError_t launch_slice(const SampleJob &j, const LaunchCfg &cfg, cudaStream_t 
         return launch_slice_as<4, 256, 2, EVAL>(j, 4 * t, t, 4 * t, st);
     }
     const int64_t sms = cfg.sms;
-    if (j.B <= sms * 512) {
-        const int shots = j.B <= sms * 128 ? 128 : j.B <= sms * 256 ? 256 : 512;
+    // (launches of one call overlap: their shape is that of the call's shots, up
+    // to the two-per-SM width, which the launches in flight fill together)
+    const int64_t n = cfg.call_shots > 0 ? std::min(cfg.call_shots, 2 * sms * 1024) : j.B;
+    if (n <= sms * 512) {
+        const int shots = n <= sms * 128 ? 128 : n <= sms * 256 ? 256 : 512;
         return launch_slice_as<1, 512, 1, EVAL>(j, shots, 512, shots, st);
     }
-    if (j.B <= sms * 1024) return launch_slice_as<4, 512, 1, EVAL>(j, 1024, 512, 1024, st);
-    const bool wide = j.B > 2 * sms * 1024;
+    if (n <= sms * 1024) return launch_slice_as<4, 512, 1, EVAL>(j, 1024, 512, 1024, st);
+    const bool wide = n > 2 * sms * 1024;
     const int shots = wide ? 2048 : 1024;
     // equal tiles: a last wave that is nearly empty costs as much as a full one
-    const int64_t waves = (j.B + 2 * sms * shots - 1) / (2 * sms * shots);
-    const int64_t want = (j.B + waves * 2 * sms - 1) / (waves * 2 * sms);
+    const int64_t all = cfg.call_shots > 0 ? cfg.call_shots : j.B;
+    const int64_t waves = (all + 2 * sms * shots - 1) / (2 * sms * shots);
+    const int64_t want = (all + waves * 2 * sms - 1) / (waves * 2 * sms);
     const int tile = (int)((want + 63) / 64 * 64);
     if (wide) return launch_slice_as<8, 256, 2, EVAL>(j, shots, 256, tile, st);
     return launch_slice_as<4, 256, 2, EVAL>(j, shots, 256, tile, st);

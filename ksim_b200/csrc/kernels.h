@@ -60,6 +60,7 @@ struct LaunchCfg {
     int slot_bytes = 16384;
     int sliced = 0;         // run the sliced stream (its own staging)
     int slice_threads = 0;  // its threads per CTA (0: tile shape from the shots)
+    int64_t call_shots = 0; // shots of the whole call when this launch is one of several that run together
     int sms = 148;          // SMs of the device
     int paths = 0;       // term paths the program uses: 0 all, 1 32-bit only, 2 32-bit and hybrid
                          // (the kernels compiled without the others)
