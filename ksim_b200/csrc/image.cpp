@@ -43,22 +43,26 @@ constexpr int kWords[] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 16};
 
 void put32(std::vector<uint8_t> &b, uint32_t v)
 {
-    uint8_t t[4];
-    std::memcpy(t, &v, 4);
-    b.insert(b.end(), t, t + 4);
+    const size_t n = b.size();
+    b.resize(n + 4);
+    std::memcpy(&b[n], &v, 4);
 }
 void put64(std::vector<uint8_t> &b, uint64_t v)
 {
-    uint8_t t[8];
-    std::memcpy(t, &v, 8);
-    b.insert(b.end(), t, t + 8);
+    const size_t n = b.size();
+    b.resize(n + 8);
+    std::memcpy(&b[n], &v, 8);
 }
 
 // sigma_k(z) for the embedding w -> e^{i k pi/4}.
 std::complex<double> embed(const int64_t z[4], int k)
 {
-    const double th = k * M_PI / 4;
-    const std::complex<double> w(std::cos(th), std::sin(th));
+    static const std::complex<double> kRoot[8] = {
+        {std::cos(0 * M_PI / 4), std::sin(0 * M_PI / 4)}, {std::cos(1 * M_PI / 4), std::sin(1 * M_PI / 4)},
+        {std::cos(2 * M_PI / 4), std::sin(2 * M_PI / 4)}, {std::cos(3 * M_PI / 4), std::sin(3 * M_PI / 4)},
+        {std::cos(4 * M_PI / 4), std::sin(4 * M_PI / 4)}, {std::cos(5 * M_PI / 4), std::sin(5 * M_PI / 4)},
+        {std::cos(6 * M_PI / 4), std::sin(6 * M_PI / 4)}, {std::cos(7 * M_PI / 4), std::sin(7 * M_PI / 4)}};
+    const std::complex<double> w = kRoot[k & 7];
     return (double)z[0] + (double)z[1] * w + (double)z[2] * (w * w) + (double)z[3] * std::conj(w);
 }
 
@@ -93,7 +97,14 @@ struct Bits {
 bool pack_mask(const uint8_t *row, int P, int W, uint64_t *out)
 {
     for (int w = 0; w < W; ++w) out[w] = 0;
-    for (int j = 0; j < P; ++j) {
+    int j = 0;
+    for (; j + 8 <= P; j += 8) {  // eight bytes at once: byte k's low bit to bit k
+        uint64_t x;
+        std::memcpy(&x, row + j, 8);
+        if (x & ~0x0101010101010101ull) return false;
+        out[j >> 6] |= (x * 0x0102040810204080ull >> 56) << (j & 63);
+    }
+    for (; j < P; ++j) {
         const uint8_t b = row[j];
         if (b > 1) return false;
         out[j >> 6] |= (uint64_t)b << (j & 63);
@@ -107,6 +118,57 @@ bool all_zero(const uint64_t *m, int W)
         if (m[w]) return false;
     return true;
 }
+
+}  // namespace
+
+namespace {
+
+// A PhasePairs factor by its phases: valuation and log2 of its norm bound.
+struct FactorTable {
+    uint32_t v[8][8];
+    double lf[8][8];
+    FactorTable()
+    {
+        for (int a = 0; a < 8; ++a)
+            for (int b = 0; b < 8; ++b) {
+                int64_t f[4];
+                phase_pair(a, b, f);
+                v[a][b] = zw_valuation(f);
+                lf[a][b] = v[a][b] == NU_ZERO ? 0.0 : std::log2(max_embed(f)) + 1e-12;
+            }
+    }
+};
+
+// Products of two factors, by the columns' classes (4 ja + jb; the second may
+// be 16, the factor 1 of an odd last column) and their four sign bits.
+struct PairEntry {
+    uint32_t v1, v2;
+    int64_t pc[4];
+    double l12;  // log2 bound of the product (unless zero)
+};
+struct PairTable {
+    std::vector<PairEntry> e;
+    PairTable() : e(16 * 17 * 16)
+    {
+        for (int c1 = 0; c1 < 16; ++c1)
+            for (int c2 = 0; c2 < 17; ++c2)
+                for (uint32_t c = 0; c < 16; ++c) {
+                    int64_t f1[4], f2[4] = {1, 0, 0, 0};
+                    phase_pair((int)((c1 >> 2) | ((c & 1u) << 2)), (int)((c1 & 3) | ((c >> 1 & 1u) << 2)), f1);
+                    if (c2 < 16)
+                        phase_pair((int)((c2 >> 2) | ((c >> 2 & 1u) << 2)), (int)((c2 & 3) | ((c >> 3) << 2)), f2);
+                    PairEntry &x = e[(size_t)((c1 * 17 + c2) * 16) + c];
+                    x.v1 = zw_valuation(f1);
+                    x.v2 = zw_valuation(f2);
+                    const Zu a = {(uint64_t)f1[0], (uint64_t)f1[1], (uint64_t)f1[2], (uint64_t)f1[3]};
+                    const Zu b = {(uint64_t)f2[0], (uint64_t)f2[1], (uint64_t)f2[2], (uint64_t)f2[3]};
+                    const Zu pr = zmul(a, b);
+                    x.pc[0] = (int64_t)pr.a; x.pc[1] = (int64_t)pr.b; x.pc[2] = (int64_t)pr.c; x.pc[3] = (int64_t)pr.d;
+                    x.l12 = x.v1 == NU_ZERO || x.v2 == NU_ZERO ? 0.0 : std::log2(max_embed(x.pc)) + 1e-12;
+                }
+    }
+    const PairEntry &at(int c1, int c2, uint32_t c) const { return e[(size_t)((c1 * 17 + c2) * 16) + c]; }
+};
 
 }  // namespace
 
@@ -218,8 +280,10 @@ int build_image(const ksim_graph_desc *gs, int n_graphs, int F, HostImage &img, 
     std::vector<uint8_t> &out = img.bytes;
     out.resize(sizeof(GraphDir) * (size_t)n_graphs, 0);
 
+    std::vector<std::vector<uint16_t>> lists(32);  // a block's rows as set bits
+    static const FactorTable factors;
+    static const PairTable pairs;
     std::vector<uint64_t> mask(2 * W);
-    std::vector<uint8_t> zero_row;
 
     for (int k = 0; k < n_graphs; ++k) {
         const ksim_graph_desc &g = gs[k];
@@ -437,11 +501,10 @@ int build_image(const ksim_graph_desc *gs, int n_graphs, int F, HostImage &img, 
                 // iff nu >= 4 (a zero factor ends the term)
                 std::map<uint32_t, double> next;
                 for (uint32_t combo = 0; combo < 4; ++combo) {  // combo = raw pa | pb << 1
-                    int64_t f[4];
-                    phase_pair((int)(ac ^ ((combo & 1u) << 2)), (int)(bc ^ ((combo >> 1) << 2)), f);
-                    const uint32_t v = zw_valuation(f);
+                    const uint32_t fa = ac ^ ((combo & 1u) << 2), fb = bc ^ ((combo >> 1) << 2);
+                    const uint32_t v = factors.v[fa][fb];
                     if (v == NU_ZERO) continue;
-                    const double lf = std::log2(max_embed(f)) + 1e-12;
+                    const double lf = factors.lf[fa][fb];
                     for (const auto &sv : ph_state) {
                         double x = sv.second + lf;
                         ref_max = std::max(ref_max, x);
@@ -474,20 +537,13 @@ int build_image(const ksim_graph_desc *gs, int n_graphs, int F, HostImage &img, 
             // exact points are the unhalved pair products, then the end.  Pair tables: the 16
             // products F F' by folded signs, and the step table of the pair's
             // halvings (see pair_step below).
-            auto ph_factor = [&](size_t col, uint32_t k, int64_t f[4]) {
-                phase_pair((int)(ph_j[col].first | ((k & 1u) << 2)), (int)(ph_j[col].second | ((k >> 1) << 2)), f);
-            };
             // (an odd last column pairs with the factor 1: valuation 0)
             const size_t n_pair = ((size_t)n_ph + 1) / 2;
             std::vector<uint8_t> pair_tab(64 * n_pair, 0);
             std::vector<uint8_t> pair_step(256 * n_pair, 0);
             bool pair_ok = true;
-            auto ph_factor2 = [&](size_t col, uint32_t k, int64_t f[4]) {
-                if (col < (size_t)n_ph) {
-                    ph_factor(col, k, f);
-                } else {
-                    f[0] = 1; f[1] = 0; f[2] = 0; f[3] = 0;
-                }
+            auto ph_class = [&](size_t col) {
+                return col < (size_t)n_ph ? (int)(4 * ph_j[col].first + ph_j[col].second) : 16;
             };
             {
                 std::map<uint32_t, double> fs;
@@ -506,11 +562,8 @@ int build_image(const ksim_graph_desc *gs, int n_graphs, int F, HostImage &img, 
                         if (sv.first >= NU_DEAD) pair_ok = false;
                     const uint32_t second = 2 * q + 1 < (size_t)n_ph ? 1u : 0u;
                     for (uint32_t c = 0; c < 16; ++c) {
-                        int64_t f1[4], f2[4];
-                        ph_factor2(2 * q, c & 3u, f1);
-                        ph_factor2(2 * q + 1, c >> 2, f2);
-                        const uint32_t v1 = std::min<uint32_t>(zw_valuation(f1), 15u);
-                        const uint32_t v2 = std::min<uint32_t>(zw_valuation(f2), 15u);
+                        const PairEntry &pe = pairs.at(ph_class(2 * q), ph_class(2 * q + 1), c);
+                        const uint32_t v1 = std::min<uint32_t>(pe.v1, 15u), v2 = std::min<uint32_t>(pe.v2, 15u);
                         pair_step[256 * q + 16 * c + NU_DEAD] = (uint8_t)(NU_DEAD << 2);
                         for (uint32_t nu0 = 0; nu0 < NU_DEAD; ++nu0) {
                             uint32_t alive = v1 != 15 ? 1u : 0u;
@@ -526,20 +579,15 @@ int build_image(const ksim_graph_desc *gs, int n_graphs, int F, HostImage &img, 
                     }
                     std::map<uint32_t, double> next;
                     for (uint32_t c = 0; c < 16; ++c) {
-                        int64_t f1[4], f2[4];
-                        ph_factor2(2 * q, c & 3u, f1);
-                        ph_factor2(2 * q + 1, c >> 2, f2);
-                        const Zu a = {(uint64_t)f1[0], (uint64_t)f1[1], (uint64_t)f1[2], (uint64_t)f1[3]};
-                        const Zu b = {(uint64_t)f2[0], (uint64_t)f2[1], (uint64_t)f2[2], (uint64_t)f2[3]};
-                        const Zu pr = zmul(a, b);
-                        const int64_t pc[4] = {(int64_t)pr.a, (int64_t)pr.b, (int64_t)pr.c, (int64_t)pr.d};
+                        const PairEntry &pe = pairs.at(ph_class(2 * q), ph_class(2 * q + 1), c);
+                        const int64_t *pc = pe.pc;
                         for (int i = 0; i < 4; ++i) {
                             if (pc[i] < -128 || pc[i] > 127) pair_ok = false;
                             pair_tab[64 * q + 4 * c + (size_t)i] = (uint8_t)(int8_t)pc[i];
                         }
-                        const uint32_t v1 = zw_valuation(f1), v2 = zw_valuation(f2);
+                        const uint32_t v1 = pe.v1, v2 = pe.v2;
                         if (v1 == NU_ZERO || v2 == NU_ZERO) continue;
-                        const double l12 = std::log2(max_embed(pc)) + 1e-12;
+                        const double l12 = pe.l12;
                         for (const auto &sv : fs) {
                             double x = sv.second + l12;
                             fast_max = std::max(fast_max, x);
@@ -738,7 +786,7 @@ int build_image(const ksim_graph_desc *gs, int n_graphs, int F, HostImage &img, 
                 nb = (uint32_t)((rows.size() + 31) / 32);
                 const uint16_t zero_off = (uint16_t)(8 * 64 * W);
                 for (uint32_t b = 0; b < nb; ++b) {
-                    std::vector<std::vector<uint16_t>> lists(32);
+                    for (std::vector<uint16_t> &l : lists) l.clear();
                     size_t n_iter = 0;  // index slots per row, rounded up to pairs
                     uint32_t masks[7] = {0, 0, 0, 0, 0, 0, 0};
                     for (int r = 0; r < 32; ++r) {
@@ -748,19 +796,21 @@ int build_image(const ksim_graph_desc *gs, int n_graphs, int F, HostImage &img, 
                             if ((role[ri] >> k) & 1u) masks[k] |= 1u << r;
                         const std::vector<uint64_t> &m = *rows[ri];
                         for (int w = 0; w < W; ++w)
-                            for (int k = 0; k < 64; ++k)
-                                if ((m[w] >> k) & 1u) lists[r].push_back((uint16_t)(8 * (64 * w + k)));
+                            for (uint64_t x = m[w]; x; x &= x - 1)
+                                lists[r].push_back((uint16_t)(8 * (64 * w + __builtin_ctzll(x))));
                         n_iter = std::max(n_iter, lists[r].size());
                     }
                     n_iter = (n_iter + 1) & ~size_t(1);
                     sum_iter += (uint32_t)n_iter;
                     put32(body, (uint32_t)(n_iter / 2));
                     for (int k = 0; k < 7; ++k) put32(body, masks[k]);
+                    size_t at = body.size();
+                    body.resize(at + 64 * n_iter);
                     for (size_t i = 0; i < n_iter; i += 2)
-                        for (int r = 0; r < 32; ++r) {
-                            const uint16_t o0 = i < lists[r].size() ? lists[r][i] : zero_off;
-                            const uint16_t o1 = i + 1 < lists[r].size() ? lists[r][i + 1] : zero_off;
-                            put32(body, (uint32_t)o0 | ((uint32_t)o1 << 16));
+                        for (int r = 0; r < 32; ++r, at += 4) {
+                            const uint16_t o[2] = {i < lists[r].size() ? lists[r][i] : zero_off,
+                                                   i + 1 < lists[r].size() ? lists[r][i + 1] : zero_off};
+                            std::memcpy(&body[at], o, 4);
                         }
                 }
             }

@@ -64,6 +64,19 @@ bool reduce(El &x)
     return true;
 }
 
+// x lambda w^6 = x (w^5 + w^6 + w^7)  (lambda = 1 + w + conj w).
+El step_lambda(const El &x)
+{
+    const i128 a = x.c[0], b = x.c[1], c = x.c[2], d = x.c[3];
+    El r;
+    r.c[0] = b + c - d;
+    r.c[1] = c - a - d;
+    r.c[2] = -(a + b + d);
+    r.c[3] = a + b + c;
+    r.e = x.e;
+    return r;
+}
+
 bool same(const El &x, const El &y) { return x.e == y.e && std::equal(x.c, x.c + 4, y.c); }
 
 // Complex value of x 2^(x.e + p2) as the reference casts it (zx_eval.hpp:
@@ -76,8 +89,16 @@ void cast(const El &x, int64_t p2, double &re, double &im)
     const double s1 = B + D, s2 = B - D;
     const double t1 = s1 * SQh, t2 = s2 * SQh;
     const int n = (int)std::max<int64_t>(-4000, std::min<int64_t>(4000, p2 + x.e));
-    re = std::ldexp(A + t1, n);
-    im = std::ldexp(C + t2, n);
+    if (n >= -1022 && n <= 1023) {  // one product with the power of two, as the reference's
+        const uint64_t bits = (uint64_t)(n + 1023) << 52;
+        double scale;
+        std::memcpy(&scale, &bits, 8);
+        re = (A + t1) * scale;
+        im = (C + t2) * scale;
+    } else {
+        re = std::ldexp(A + t1, n);
+        im = std::ldexp(C + t2, n);
+    }
 }
 
 // A parity row: its parameters and whether its parity is complemented.
@@ -90,7 +111,14 @@ Row make_row(const uint8_t *m, int P, uint32_t inv)
 {
     Row r;
     r.inv = inv & 1u;
-    for (int j = 0; j < P; ++j)
+    r.bits.reserve(8);
+    int j = 0;
+    for (; j + 8 <= P; j += 8) {  // most of a mask is zero
+        uint64_t x;
+        std::memcpy(&x, m + j, 8);
+        for (; x; x &= x - 1) r.bits.push_back((uint16_t)(j + (__builtin_ctzll(x) >> 3)));
+    }
+    for (; j < P; ++j)
         if (m[j]) r.bits.push_back((uint16_t)j);
     return r;
 }
@@ -115,7 +143,7 @@ enum Kind { K_ZERO, K_TWO, K_22, K_P, K_Q, K_B, K_L0, K_L1 };
 const El kTwo = el(2, 0, 0, 0), k22 = el(2, 0, 2, 0), kP = el(1, 2, -1, 0), kQ = el(1, -2, -1, 0),
          kB = el(1, 0, 1, 0), kKappa = el(1, -1, 1, -1), kLam = el(1, 1, 0, 1), kLamInv = el(-1, 1, 0, 1);
 
-bool classify(int a, int b, Kind &kind, int &k)
+bool find_kind(int a, int b, Kind &kind, int &k)
 {
     const El one = el(1, 0, 0, 0);
     const El u = rot(one, a), v = rot(one, b), x = rot(one, a + b);
@@ -135,6 +163,26 @@ bool classify(int a, int b, Kind &kind, int &k)
                 return true;
             }
     return false;
+}
+
+// The kinds of all 64 (alpha, beta) pairs.
+struct KindTable {
+    Kind kind[8][8];
+    int k[8][8];
+    bool ok[8][8];
+    KindTable()
+    {
+        for (int a = 0; a < 8; ++a)
+            for (int b = 0; b < 8; ++b) ok[a][b] = find_kind(a, b, kind[a][b], k[a][b]);
+    }
+};
+
+bool classify(int a, int b, Kind &kind, int &k)
+{
+    static const KindTable t;
+    kind = t.kind[a][b];
+    k = t.k[a][b];
+    return t.ok[a][b];
 }
 
 // A term's rows by role.
@@ -178,6 +226,7 @@ Group make_group(const Row *const *rows, int n, int zero_row)
     size_t slots = 1;
     for (int r = 0; r < n; ++r) slots = std::max(slots, rows[r]->bits.size());
     g.slots = (uint32_t)slots;
+    g.bytes.reserve((size_t)n * (4 + (slots + 3) / 4 * 4));
     for (int r = 0; r < n; ++r) g.bytes.insert(g.bytes.end(), 4, rows[r]->inv ? 0xFFu : 0u);
     for (size_t i = 0; i < slots; i += 4)
         for (int r = 0; r < n; ++r)
@@ -198,8 +247,10 @@ std::vector<Group> make_groups(const std::vector<Row> &rows, int step, const Row
         for (int k = 0; k < step; ++k) n = std::max(n, rows[i + (size_t)k].bits.size());
         return n;
     };
-    std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) { return weight(x) > weight(y); });
+    if (order.size() > 1)
+        std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) { return weight(x) > weight(y); });
     std::vector<const Row *> seq;
+    seq.reserve(rows.size() + 3);
     for (size_t i : order)
         for (int k = 0; k < step; ++k) seq.push_back(&rows[i + (size_t)k]);
     while (seq.size() % SLICE_GROUP) seq.push_back(step == 1 || (seq.size() & 1u) ? &zero : &pad0);
@@ -387,7 +438,6 @@ bool build_term(const ksim_graph_desc &g, int t, int zero_row, TermOutBytes &o)
         ar = g.pf_approx_f32[2 * (size_t)t];
         ai = g.pf_approx_f32[2 * (size_t)t + 1];
     }
-    const El lam6 = rot(kLam, 6);  // one X step: lambda w^6
     for (size_t ci = 0; ci < cls.size(); ++ci) {
         const int y = cls[ci].first, z = cls[ci].second;
         El v = base;
@@ -397,7 +447,7 @@ bool build_term(const ksim_graph_desc &g, int t, int zero_row, TermOutBytes &o)
         }
         for (int X = 0; X <= nx; ++X) {
             if (X) {
-                v = mul(v, lam6);
+                v = step_lambda(v);
                 if (!reduce(v)) return false;
             }
             for (i128 c : v.c)
