@@ -570,6 +570,13 @@ ksim_status ksim_program_create(ksim_component *const *comps, int32_t n_comps, c
         if (e == cudaSuccess) e = cudaMalloc(&part.d_cols, sizeof(int32_t) * std::max(n, 1));
         if (e == cudaSuccess && n > 0)
             e = cudaMemcpy(part.d_cols, dest.data() + off, sizeof(int32_t) * n, cudaMemcpyHostToDevice);
+        auto first_of_run = [](const int32_t *x, int m) {
+            for (int i = 1; i < m; ++i)
+                if (x[i] != x[0] + i) return -1;
+            return m > 0 ? x[0] : 0;
+        };
+        part.sel0 = first_of_run(f_selection[k], F);
+        part.col0 = first_of_run(dest.data() + off, n);
         p->parts.push_back(part);
         if (e != cudaSuccess) {
             ksim_program_destroy(p.release());
@@ -635,13 +642,13 @@ ksim_status ksim_program_job(const ksim_program *p, int32_t k, const uint8_t *d_
     const ProgramPart &part = p->parts[k];
     ksim_batch_job j = {};
     j.comp = part.comp;
-    j.d_f = d_f;
+    j.d_f = part.sel0 > 0 && d_f ? d_f + part.sel0 : d_f;
     j.f_stride = f_stride;
-    j.d_f_sel = part.d_sel;
+    j.d_f_sel = part.sel0 >= 0 ? nullptr : part.d_sel;
     j.d_out = d_out;
     j.out_stride = p->n_outputs;
-    j.out_col0 = 0;
-    j.d_out_cols = part.d_cols;
+    j.out_col0 = std::max(part.col0, 0);
+    j.d_out_cols = part.col0 >= 0 ? nullptr : part.d_cols;
     j.B = B;
     j.shot_offset = shot_offset;
     j.seed = seed + 0x9E37ull * (uint64_t)k;
@@ -680,12 +687,14 @@ static ksim_status program_launch(ksim_program *p, const uint8_t *d_f_params, in
         ksim_status st = component_job(c, cfg, j);
         if (st != KSIM_OK) return st;
         j.rng_mode = rng_mode;
-        j.f = d_f_params;
+        const ProgramPart &part = p->parts[k];
+        j.f = part.sel0 > 0 ? d_f_params + part.sel0 : d_f_params;
         j.f_stride = n_f_cols;
-        j.f_sel = p->parts[k].d_sel;
+        j.f_sel = part.sel0 >= 0 ? nullptr : part.d_sel;
         j.out = d_out;
         j.out_stride = p->n_outputs;
-        j.out_cols = p->parts[k].d_cols;
+        j.out_col0 = std::max(part.col0, 0);
+        j.out_cols = part.col0 >= 0 ? nullptr : part.d_cols;
         j.B = B;
         j.shot_offset = shot_offset;
         j.seed = seed + 0x9E37ull * (uint64_t)k;

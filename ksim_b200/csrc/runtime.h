@@ -67,6 +67,9 @@ struct ProgramPart {
     ksim_component *comp = nullptr;
     int32_t *d_sel = nullptr;   // f_selection on the device
     int32_t *d_cols = nullptr;  // destination output column of each component output
+    // first column where the selection / the destinations are consecutive, else
+    // -1 (kernels then take a pointer instead of the column list)
+    int32_t sel0 = -1, col0 = -1;
 };
 
 #ifndef KSIM_HOST_STREAMS

@@ -340,13 +340,14 @@ ksim_status admit(ksim_server *s, ServeRequest *r)
         ksim_status st = component_job(c, s->lcfg, J.j);
         if (st != KSIM_OK) return st;
         J.j.rng_mode = r->rng_mode;
-        J.j.f = d_f;
+        const ProgramPart &part = p->parts[k];
+        J.j.f = part.sel0 > 0 ? d_f + part.sel0 : d_f;
         J.j.f_stride = r->n_f_cols;
-        J.j.f_sel = p->parts[k].d_sel;
+        J.j.f_sel = part.sel0 >= 0 ? nullptr : part.d_sel;
         J.j.out = d_out;
         J.j.out_stride = p->n_outputs;
-        J.j.out_col0 = 0;
-        J.j.out_cols = p->parts[k].d_cols;
+        J.j.out_col0 = std::max(part.col0, 0);
+        J.j.out_cols = part.col0 >= 0 ? nullptr : part.d_cols;
         J.j.amp = nullptr;
         J.j.B = r->B;
         J.j.shot_offset = 0;

@@ -140,6 +140,17 @@ __device__ __forceinline__ void slice_add(W2 (&c)[N], int o)
     }
 }
 
+// 4 x 4 byte transpose: byte k of word i to byte i of word k.
+__device__ __forceinline__ void transpose4(uint32_t (&x)[4])
+{
+    const uint32_t a0 = __byte_perm(x[0], x[1], 0x5140), a1 = __byte_perm(x[0], x[1], 0x7362);
+    const uint32_t b0 = __byte_perm(x[2], x[3], 0x5140), b1 = __byte_perm(x[2], x[3], 0x7362);
+    x[0] = __byte_perm(a0, b0, 0x5410);
+    x[1] = __byte_perm(a0, b0, 0x7632);
+    x[2] = __byte_perm(a1, b1, 0x5410);
+    x[3] = __byte_perm(a1, b1, 0x7632);
+}
+
 // Eight planes of 32 shots to 32 bytes: word r, byte j of q holds bit 8 j + r
 // of every plane, plane k in its bit k.  Stored as the 32 bytes at o.
 __device__ __forceinline__ void slice_store(uint32_t (&p)[8], uint8_t *o)
@@ -435,45 +446,79 @@ __device__ __forceinline__ bool slice_tile(const SampleJob &j, const int64_t s0,
         }
     };
 
-    // parameter rows: the f bits (four bytes at a time where rows allow it),
-    // outputs zero for graph 0, the zero row
-    const bool vec = !j.f_sel && ((((uintptr_t)j.f) | (uintptr_t)j.f_stride) & 3u) == 0;
+    // Parameter rows p .. p + 3 (those below F) from each shot's four bytes.  S =
+    // 4, 8: byte transposes give each thread a parameter's bits of four shots in
+    // the low bits of four bytes; shifted to their places they are combined over
+    // the word's lanes, each of the first four ending up with one parameter.
+    auto put_rows4 = [&](int p, uint32_t (&x)[S]) {
+        if (S == 1) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t word = __ballot_sync(~0u, x[0] & (1u << (8 * i)));
+                if (mine && r == 0 && p + i < F) *(uint32_t *)(smem + (p + i) * SLICE_ROW + wcol) = word;
+            }
+        } else {
+            uint32_t t[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+            for (int h = 0; h < S / 4; ++h) {
+                uint32_t y[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) y[k] = x[(4 * h + k) % S] & 0x01010101u;
+                transpose4(y);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) t[i] |= y[i] << (r + 4 * h);
+            }
+            const bool o1 = r & 1, o2 = r & 2;
+            const uint32_t s0 = o1 ? t[0] : t[2], s1 = o1 ? t[1] : t[3];
+            uint32_t u0 = o1 ? t[2] : t[0], u1 = o1 ? t[3] : t[1];
+            u0 |= __shfl_xor_sync(~0u, s0, 1);
+            u1 |= __shfl_xor_sync(~0u, s1, 1);
+            uint32_t v = o2 ? u1 : u0;
+            v |= __shfl_xor_sync(~0u, o2 ? u0 : u1, 2);
+            if (S == 4) v |= __shfl_xor_sync(~0u, v, 4);
+            const int row = p + 2 * (r & 1) + ((r >> 1) & 1);
+            if (mine && r < 4 && row < F) *(uint32_t *)(smem + row * SLICE_ROW + wcol) = v;
+        }
+    };
+
+    // parameter rows: the f bits (16 or 4 bytes of a row at a time where rows
+    // allow it), outputs zero for graph 0, the zero row
     int p0 = 0;
-    if (vec) {
-        for (; p0 + 8 <= F; p0 += 8) {
-            uint32_t x[S][2];
+    if (!j.f_sel && ((((uintptr_t)j.f) | (uintptr_t)j.f_stride) & 15u) == 0) {
+        for (; p0 + 16 <= F; p0 += 16) {
+            uint4 x[S];
 #pragma unroll
             for (int k = 0; k < S; ++k)
+                x[k] = ((act >> k) & 1u) ? ldj<CG>((const uint4 *)(j.f + sh_of(k) * j.f_stride + p0))
+                                         : make_uint4(0u, 0u, 0u, 0u);
+            uint32_t y[S];
+#define KSIM_ROWS4(M, Q)                                       \
+    _Pragma("unroll") for (int k = 0; k < S; ++k) y[k] = x[k].M; \
+    put_rows4(p0 + 4 * Q, y);
+            KSIM_ROWS4(x, 0) KSIM_ROWS4(y, 1) KSIM_ROWS4(z, 2) KSIM_ROWS4(w, 3)
+#undef KSIM_ROWS4
+        }
+    }
+    if (!j.f_sel && ((((uintptr_t)j.f) | (uintptr_t)j.f_stride) & 3u) == 0) {
+        for (; p0 + 4 <= F; p0 += 4) {
+            uint32_t x[S];
 #pragma unroll
-                for (int h = 0; h < 2; ++h)
-                    x[k][h] = ((act >> k) & 1u)
-                                  ? ldj<CG>((const uint32_t *)(j.f + sh_of(k) * j.f_stride + p0) + h) : 0u;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                bool b[S];
-#pragma unroll
-                for (int k = 0; k < S; ++k) b[k] = x[k][i >> 2] & (1u << (8 * (i & 3)));
-                put_row(p0 + i, b);
-            }
+            for (int k = 0; k < S; ++k)
+                x[k] = ((act >> k) & 1u) ? ldj<CG>((const uint32_t *)(j.f + sh_of(k) * j.f_stride + p0)) : 0u;
+            put_rows4(p0, x);
         }
     }
     for (; p0 < F; p0 += 4) {
-        uint8_t x[S][4];
+        uint32_t x[S] = {};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int p = min(p0 + i, F - 1);
             const int col = j.f_sel ? ldj<CG>(j.f_sel + p) : p;
 #pragma unroll
             for (int k = 0; k < S; ++k)
-                x[k][i] = ((act >> k) & 1u) ? ldj<CG>(j.f + sh_of(k) * j.f_stride + col) : (uint8_t)0;
+                if ((act >> k) & 1u) x[k] |= (uint32_t)ldj<CG>(j.f + sh_of(k) * j.f_stride + col) << (8 * i);
         }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            bool b[S];
-#pragma unroll
-            for (int k = 0; k < S; ++k) b[k] = x[k][i] & 1u;
-            if (p0 + i < F) put_row(p0 + i, b);
-        }
+        put_rows4(p0, x);
     }
     auto fill_rows = [&](int from, int to, uint32_t x) {
         for (int i = tid; i < (to - from) * (SLICE_ROW / 4); i += nthr) {
@@ -626,13 +671,53 @@ __device__ __forceinline__ bool slice_tile(const SampleJob &j, const int64_t s0,
     g += (uint32_t)nch;
     if (EVAL >= 0) return true;
 
-    for (int i = 0; i < j.n_out && mine; ++i) {
-        const uint32_t x = *(const uint32_t *)(smem + (F + i) * SLICE_ROW + wcol) >> r;
-        const int64_t col = j.out_cols ? (int64_t)ldj<CG>(j.out_cols + i) : j.out_col0 + i;
+    // output rows, eight or four columns at once where they are contiguous and
+    // aligned
+    if (mine) {
+        auto word_of = [&](int i) { return *(const uint32_t *)(smem + (F + i) * SLICE_ROW + wcol) >> r; };
+        const uintptr_t place = j.out_cols ? 1u : (uintptr_t)(j.out + j.out_col0) | (uintptr_t)j.out_stride;
+        int i = 0;
+        if (S > 1 && (place & 3u) == 0) {
+            uint8_t *out = j.out + j.out_col0;
+            const bool pairs = (place & 7u) == 0;
+            while (i + 4 <= j.n_out) {
+                const bool two = pairs && i + 8 <= j.n_out;
+                uint32_t x[2][4];
 #pragma unroll
-        for (int k = 0; k < S; ++k)
-            if ((act >> k) & 1u)
-                j.out[sh_of(k) * j.out_stride + col] = (uint8_t)((x >> (S == 8 ? 8 * (k & 3) + 4 * (k >> 2) : 8 * k)) & 1u);
+                for (int k = 0; k < 4; ++k) {
+                    x[0][k] = word_of(i + k);
+                    x[1][k] = two ? word_of(i + 4 + k) : 0u;
+                }
+#pragma unroll
+                for (int h = 0; h < (S + 3) / 4; ++h) {
+                    uint32_t y[2][4];
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) y[q][k] = (x[q][k] >> (4 * h)) & 0x01010101u;
+                        transpose4(y[q]);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const int sh = (4 * h + k) % S;
+                        if (!((act >> sh) & 1u)) continue;
+                        uint8_t *o = out + sh_of(sh) * j.out_stride + i;
+                        if (two) *(uint2 *)o = make_uint2(y[0][k], y[1][k]);
+                        else *(uint32_t *)o = y[0][k];
+                    }
+                }
+                i += two ? 8 : 4;
+            }
+        }
+        for (; i < j.n_out; ++i) {
+            const uint32_t x = word_of(i);
+            const int64_t col = j.out_cols ? (int64_t)ldj<CG>(j.out_cols + i) : j.out_col0 + i;
+#pragma unroll
+            for (int k = 0; k < S; ++k)
+                if ((act >> k) & 1u)
+                    j.out[sh_of(k) * j.out_stride + col] =
+                        (uint8_t)((x >> (S == 8 ? 8 * (k & 3) + 4 * (k >> 2) : 8 * k)) & 1u);
+        }
     }
     if (flags) atomicOr(j.status, flags);
     return true;
