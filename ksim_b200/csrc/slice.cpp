@@ -366,7 +366,7 @@ bool build_term(const ksim_graph_desc &g, int t, int zero_row, TermOutBytes &o)
     }
     R.k0 += (R.w4.inv ? 4 : 0) + (int)(g.pf_phase_idx[t] & 7u);
     const int n9 = (int)R.n9.size() / 2, nx = n1 + n3 + R.n_8;
-    if (nx > 127 || n9 > 15) return false;
+    if (nx > 126 || n9 > 15) return false;
     const bool wide = n9 > 4, even = R.w1.empty();
 
     SliceTerm &d = o.d;
@@ -389,9 +389,9 @@ bool build_term(const ksim_graph_desc &g, int t, int zero_row, TermOutBytes &o)
     // the pair products enter K's bit 2 or its other half S: they go to
     // whichever half of the term has less to do
     double cost_k = 0, cost_x = 0;
-    for (int i : {SQ_KILL, SQ_W1, SQ_W2, SQ_W4, SQ_N9})
+    for (int i : {SQ_W1, SQ_W2, SQ_W4, SQ_N9})
         for (const Group &x : role[i]) cost_k += x.cost();
-    for (int i : {SQ_X1, SQ_X0})
+    for (int i : {SQ_X1, SQ_X0, SQ_KILL})
         for (const Group &x : role[i]) cost_x += x.cost();
     for (Group &x : make_groups(R.pp, 2, Row(), zero_row)) {
         double &c = cost_k <= cost_x ? cost_k : cost_x;
@@ -402,7 +402,7 @@ bool build_term(const ksim_graph_desc &g, int t, int zero_row, TermOutBytes &o)
         for (Group &x : role[i]) {
             x.role = i;
             if (x.slots > 255u) return false;
-            (i < SQ_X_ROLES ? d.n_k : d.n_x) += 1;
+            (i < SQ_X1 ? d.n_k : i == SQ_X1 ? d.n_x1 : i == SQ_X0 ? d.n_x0 : d.n_xp) += 1;
             o.groups.push_back(std::move(x));
         }
 
@@ -417,7 +417,7 @@ bool build_term(const ksim_graph_desc &g, int t, int zero_row, TermOutBytes &o)
     const int n_par = even ? 1 : 2;
     const size_t xs = cls.size() * (size_t)n_par * 16;
     d.xs = (uint16_t)xs;
-    o.tab.assign(xs * (size_t)(nx + 1), 0);
+    o.tab.assign(xs * (size_t)(nx + 2), 0);
 
     base.e += R.n_two;
     for (int i = 0; i < R.n_22; ++i) base = mul(base, k22);
@@ -461,7 +461,7 @@ bool build_term(const ksim_graph_desc &g, int t, int zero_row, TermOutBytes &o)
                     re = a - b;
                     im = c + e;
                 }
-                const size_t at = (size_t)X * xs + (ci * (size_t)n_par + (size_t)r) * 16;
+                const size_t at = (size_t)(X + 1) * xs + (ci * (size_t)n_par + (size_t)r) * 16;
                 std::memcpy(&o.tab[at], &re, 8);
                 std::memcpy(&o.tab[at + 8], &im, 8);
                 w = rot1(w);

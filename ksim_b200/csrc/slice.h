@@ -50,34 +50,33 @@ constexpr int SLICE_MAX_PLANES = 16;  // result bytes per shot of a chunk's term
 constexpr int SLICE_MAX_TERMS = 8;    // of a chunk
 constexpr int SLICE_AHEAD = 2;        // chunks staged at once
 
-// A chunk starts with a zero table entry (the dead terms') and what a CTA
-// needs to know of it and of the chunk SLICE_AHEAD behind it.
+// A chunk starts with what a CTA needs to know of it and of the chunk
+// SLICE_AHEAD behind it.
 struct SliceChunk {
-    uint64_t zero[2];
     uint16_t n_terms, end_of_graph;
     uint32_t graph, ahead_bytes, ahead_off16;
 };
 constexpr int SLICE_HEAD = sizeof(SliceChunk);
-static_assert(SLICE_HEAD == 32, "SliceChunk layout");
+static_assert(SLICE_HEAD == 16, "SliceChunk layout");
 constexpr int SLICE_BIG_TABLE = 16384;  // larger tables stay in global memory
 
 enum : uint32_t { ST_WIDE = 1u, ST_BIG = 2u, ST_EVEN = 4u };
 
 // A term's result per shot, one byte a plane:
-//   X plane: X (7 bits), bit 7 the parity S of the class-1 rows;
+//   X plane: X + 1, or 0 of a dead term (7 bits), bit 7 the parity S of the
+//     class-1 rows;
 //   K plane: bits 0-5 the table column in half entries (K's bit 1, then K's
-//     bit 0 unless ST_EVEN, then the class of (y, z)), bit 6 kill, bit 7 K's
-//     bit 2 without S;
+//     bit 0 unless ST_EVEN, then the class of (y, z)), bit 7 K's bit 2
+//     without S;
 //   ST_WIDE (more than four p / q columns): a third plane y | z << 4, whose
 //     class is read from a table of 256 (the K plane then has class 0).
-// The value is table[X][class][K0] * i^(2 (K2 ^ S) + K1), each entry a complex
-// double (16 bytes); a dead term's is the zero entry at the chunk's start.
+// The value is table[X + 1][class][K0] * i^(2 (K2 ^ S) + K1), each entry a
+// complex double (16 bytes); table[0] is zero.
 
-// Roles of a term's rows, in stream order.  The K half: kill; K by weight 1,
-// 2, 4; p / q columns; weight-4 pairs.  The X half: X with and without S;
-// weight-4 pairs, into S.
-enum { SQ_KILL, SQ_W1, SQ_W2, SQ_W4, SQ_N9, SQ_PPK, SQ_X1, SQ_X0, SQ_PPX, SQ_ROLES };
-constexpr int SQ_X_ROLES = SQ_X1;  // first role of the X half
+// Roles of a term's rows, in stream order.  The K half: K by weight 1, 2, 4;
+// p / q columns; weight-4 pairs.  The X half: X with and without S; weight-4
+// pairs, into S; kill.
+enum { SQ_W1, SQ_W2, SQ_W4, SQ_N9, SQ_PPK, SQ_X1, SQ_X0, SQ_PPX, SQ_KILL, SQ_ROLES };
 
 // One term of a chunk, behind its head.  Its rows come in groups of
 // four, listed role by role as u32: bits 0-15 the group's offset in the chunk /
@@ -90,9 +89,10 @@ struct SliceTerm {
     uint16_t list_off16;  // group list (16-byte units, in the chunk)
     uint16_t lut_off16;   // ST_WIDE: 256 bytes, class of y | z << 4
     uint16_t plane;       // first result plane
-    uint16_t n_k, n_x;    // groups of the K half and of the X half
-    uint16_t pad0;
-    uint32_t pad1[3];
+    uint16_t n_k;         // groups of the K half
+    uint16_t n_x1, n_x0;  // of X with and without S,
+    uint16_t n_xp;        // of the X half's pairs and kill rows
+    uint16_t pad[5];
 };
 static_assert(sizeof(SliceTerm) == 32, "SliceTerm layout");
 

@@ -5,7 +5,7 @@
 // runs two passes:
 //   rows    a warp takes one half of a term (its K roles or its X roles): L
 //           lanes cover the tile's shots, 64 each, and the 32 / L lane groups
-//           share the quads of every role.  A lane forms parity rows as XORs
+//           share the groups of four rows of every role.  A lane forms parity rows as XORs
 //           of a few parameter words and adds them into bit-sliced counters
 //           (carry-save adders); the groups' counters are added over
 //           shuffles, and the eight result planes become one byte per shot by
@@ -59,66 +59,66 @@ __device__ __forceinline__ W2 maj(W2 x, W2 y, W2 z)
     return {(x.a & y.a) | (x.a & z.a) | (y.a & z.a), (x.b & y.b) | (x.b & z.b) | (y.b & z.b)};
 }
 
-// The N rows of a group for this lane's 64 shots.  lane8: the shared address
-// of the lane's column of the parameter rows.  A slot's address is one dot
-// product (byte k of the word times the row pitch, plus the column).
-template <int N>
-__device__ __forceinline__ void slice_rows(uint32_t entry, const uint8_t *chunk, uint32_t lane8, W2 (&r)[N])
+// The four rows of a group for this lane's 64 shots.  lane8: the shared
+// address of the lane's column of the parameter rows.  A slot's address is one
+// dot product (byte k of the word times the row pitch, plus the column).  Most
+// rows have one to four parameters: a straight path each.
+__device__ __forceinline__ W2 slice_ld(uint32_t x, int k, uint32_t lane8)
+{
+    W2 v;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.a), "=r"(v.b)
+                 : "r"(__dp4a(x, (uint32_t)SLICE_ROW << (8 * k), lane8)));
+    return v;
+}
+__device__ __forceinline__ void slice_rows(uint32_t entry, const uint8_t *chunk, uint32_t lane8, W2 (&r)[SLICE_GROUP])
 {
     const uint4 *p = (const uint4 *)(chunk + 16u * (entry & 0xFFFFu));
     int n = (int)((entry >> 16) & 0xFFu);
-    uint32_t u[N];
-    auto words = [&](uint32_t (&x)[N]) {
+    const uint4 inv4 = p[0], u4 = p[1];
+    const uint32_t inv[4] = {inv4.x, inv4.y, inv4.z, inv4.w};
+    const uint32_t u[4] = {u4.x, u4.y, u4.z, u4.w};
+    if (n == 1) {
 #pragma unroll
-        for (int i = 0; i < N; i += 4) {
-            const uint4 v = *p++;
-            x[i] = v.x; x[i + 1] = v.y; x[i + 2] = v.z; x[i + 3] = v.w;
-        }
+        for (int i = 0; i < 4; ++i) r[i] = slice_ld(u[i], 0, lane8);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) r[i] = {r[i].a ^ inv[i], r[i].b ^ inv[i]};
+        return;
+    }
+    {
+        W2 x[4], y[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] = slice_ld(u[i], 0, lane8);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) y[i] = slice_ld(u[i], 1, lane8);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) r[i] = {x[i].a ^ y[i].a ^ inv[i], x[i].b ^ y[i].b ^ inv[i]};
+    }
+    if (n == 2) return;
+    if (n == 3) {
+        W2 x[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] = slice_ld(u[i], 2, lane8);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) r[i] = r[i] ^ x[i];
+        return;
+    }
+    auto pair = [&](const uint32_t (&v)[4], int k) {
+        W2 x[4], y[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] = slice_ld(v[i], k, lane8);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) y[i] = slice_ld(v[i], k + 1, lane8);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) r[i] = r[i] ^ x[i] ^ y[i];
     };
-    words(u);
-#pragma unroll
-    for (int i = 0; i < N; ++i) r[i] = {u[i], u[i]};
-    words(u);
-    auto ld = [&](uint32_t x, int k) {
-        W2 v;
-        asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.a), "=r"(v.b)
-                     : "r"(__dp4a(x, (uint32_t)SLICE_ROW << (8 * k), lane8)));
-        return v;
-    };
-    auto one = [&](int k) {
-        W2 x[N];
-#pragma unroll
-        for (int i = 0; i < N; ++i) x[i] = ld(u[i], k);
-#pragma unroll
-        for (int i = 0; i < N; ++i) r[i] = r[i] ^ x[i];
-    };
-    auto two = [&](int k) {
-#pragma unroll
-        for (int h = 0; h < N; h += 4) {
-            W2 x[4], y[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) x[i] = ld(u[h + i], k);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) y[i] = ld(u[h + i], k + 1);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) r[h + i] = r[h + i] ^ x[i] ^ y[i];
-        }
-    };
-    for (;;) {
-        if (n == 1) {
-            one(0);
-            break;
-        }
-        two(0);
-        if (n == 2) break;
-        if (n == 3) {
-            one(2);
-            break;
-        }
-        two(2);
-        n -= 4;
-        if (n == 0) break;
-        words(u);
+    pair(u, 2);
+    for (n -= 4, p += 2; n > 0; n -= 2) {  // (unused slots name the zero row)
+        const uint4 v4 = *p;
+        const uint32_t v[4] = {v4.x, v4.y, v4.z, v4.w};
+        pair(v, 0);
+        if ((n -= 2) <= 0) break;
+        pair(v, 2);
+        ++p;
     }
 }
 
@@ -211,61 +211,94 @@ __device__ __forceinline__ void slice_add4x(W2 &x0, W2 &x1, W2 b0, W2 b1, W2 b2,
     x1 = x1 ^ t0 ^ t1;
 }
 
-// One half of a term.  Planes a[]: K half 0-2 K, 3 kill, 4-7 y, 8-11 z; X half
-// 0-6 X, 7 S.  One loop over the half's groups, so the row code exists once.
-__device__ __forceinline__ void slice_task(const uint8_t *chunk, const SliceTerm &d, bool x_half, uint8_t *planes,
-                                           int plane_bytes, const SliceLane &ln)
+// The X half of a term: planes 0-6 X + 1 (0: dead), 7 S, the parity of X's
+// count after its class-1 rows.  The halves are loops of their own, X's without
+// a look at the role: of ~3,200 warp instructions a term's rows pass took for
+// 2,048 shots, ~700 were the one loop's role dispatch and ~450 register moves
+// (606,208 shots of the 40-output program: 0.783 -> 0.711 ms).
+__device__ __forceinline__ void slice_x(const uint8_t *chunk, const SliceTerm &d, uint8_t *planes, int plane_bytes,
+                                        const SliceLane &ln)
 {
-    const uint32_t *list = (const uint32_t *)(chunk + 16 * (int)d.list_off16) + (x_half ? (int)d.n_k : 0);
-    const int n = x_half ? d.n_x : d.n_k;
-    W2 a[12];
+    const uint32_t *list = (const uint32_t *)(chunk + 16 * (int)d.list_off16) + (int)d.n_k;
+    const uint32_t one = ln.grp == 0 ? ~0u : 0u;
+    W2 a[8], kill = {0u, 0u}, s = {0u, 0u};
+    a[0] = {one, one};
 #pragma unroll
-    for (int i = 0; i < 12; ++i) a[i] = {0u, 0u};
-    bool n9 = false;
-    for (int q = ln.grp; q < n; q += ln.n_grp) {
-        const uint32_t e = list[q], role = (e >> 24) & 15u;
-        W2 r[SLICE_GROUP];
-        slice_rows<SLICE_GROUP>(e, chunk, ln.lane8, r);
-        if (role == SQ_X1 || role == SQ_X0) {
-            if (role == SQ_X1) {
-#pragma unroll
-                for (int i = 0; i < SLICE_GROUP; i += 2) a[7] = a[7] ^ r[i] ^ r[i + 1];
-            }
+    for (int i = 1; i < 8; ++i) a[i] = {0u, 0u};
+    int q = ln.grp, n = d.n_x1;
+    for (int phase = 0; phase < 2; ++phase) {
+        for (; q < n; q += ln.n_grp) {
+            W2 r[SLICE_GROUP];
+            slice_rows(list[q], chunk, ln.lane8, r);
             W2 c = slice_add4(a[0], a[1], r[0], r[1], r[2], r[3]);
-            int from = 2;
-            if (SLICE_GROUP == 8) {
-                const W2 f = slice_add4(a[0], a[1], r[SLICE_GROUP - 4], r[SLICE_GROUP - 3], r[SLICE_GROUP - 2], r[SLICE_GROUP - 1]);
-                const W2 t = maj(a[2], c, f);
-                a[2] = a[2] ^ c ^ f;
-                c = t;
-                from = 3;
-            }
 #pragma unroll
             for (int i = 2; i < 7; ++i) {
-                if (i < from) continue;
                 const W2 t = a[i] & c;
                 a[i] = a[i] ^ c;
                 c = t;
             }
-        } else if (role == SQ_PPX || role == SQ_PPK) {
-            W2 t = (r[0] & r[1]) ^ (r[2] & r[3]);
+        }
+        if (phase == 0) {
+            s = a[0];  // the parity so far, complemented by `one`
+            n += d.n_x0;
+        }
+    }
+    s = {s.a ^ one, s.b ^ one};
+    n += d.n_xp;
+    for (; q < n; q += ln.n_grp) {
+        const uint32_t e = list[q];
+        W2 r[SLICE_GROUP];
+        slice_rows(e, chunk, ln.lane8, r);
+        if (e >> 24 == SQ_PPX) {
+            s = s ^ (r[0] & r[1]);
+            s = s ^ (r[2] & r[3]);
+        } else {
+            kill = kill | r[0] | r[1];
+            kill = kill | r[2] | r[3];
+        }
+    }
+    for (int o = ln.L; o < 32; o <<= 1) {
+        s = s ^ slice_shfl(s, o);
+        kill = kill | slice_shfl(kill, o);
+        slice_add<0, 7>(a, o);
+    }
+    uint8_t *out = planes + (int)d.plane * plane_bytes;
+    slice_finish(ln, [&](int h, int word) {
+        uint32_t p[8];
+        const uint32_t live = ~slice_pick(kill, h);
 #pragma unroll
-            for (int i = 4; i < SLICE_GROUP; i += 2) t = t ^ (r[i] & r[i + 1]);
-            if (role == SQ_PPX) a[7] = a[7] ^ t;
-            else a[2] = a[2] ^ t;
-        } else if (role == SQ_W2) {
+        for (int i = 0; i < 7; ++i) p[i] = slice_pick(a[i], h) & live;
+        p[7] = slice_pick(s, h);
+        slice_store(p, out + 32 * word);
+    });
+}
+
+// The K half: planes a[0..2] K, y[] and z[] the p and q counts.
+__device__ __forceinline__ void slice_k(const uint8_t *chunk, const SliceTerm &d, uint8_t *planes, int plane_bytes,
+                                        const SliceLane &ln)
+{
+    const uint32_t *list = (const uint32_t *)(chunk + 16 * (int)d.list_off16);
+    const int n = d.n_k;
+    W2 a[3], y[4], z[4];
 #pragma unroll
-            for (int i = 0; i < SLICE_GROUP; i += 4) slice_add4x(a[1], a[2], r[i], r[i + 1], r[i + 2], r[i + 3]);
-        } else if (role == SQ_W4) {
+    for (int i = 0; i < 3; ++i) a[i] = {0u, 0u};
 #pragma unroll
-            for (int i = 0; i < SLICE_GROUP; i += 2) a[2] = a[2] ^ r[i] ^ r[i + 1];
-        } else if (role == SQ_KILL) {
-#pragma unroll
-            for (int i = 0; i < SLICE_GROUP; i += 2) a[3] = a[3] | r[i] | r[i + 1];
+    for (int i = 0; i < 4; ++i) y[i] = z[i] = {0u, 0u};
+    bool n9 = false;
+    for (int q = ln.grp; q < n; q += ln.n_grp) {
+        const uint32_t e = list[q], role = e >> 24;
+        W2 r[SLICE_GROUP];
+        slice_rows(e, chunk, ln.lane8, r);
+        if (role == SQ_PPK) {
+            a[2] = a[2] ^ (r[0] & r[1]);
+            a[2] = a[2] ^ (r[2] & r[3]);
         } else if (role == SQ_W1) {
-#pragma unroll
-            for (int i = 0; i < SLICE_GROUP; i += 4)
-                a[2] = a[2] ^ slice_add4(a[0], a[1], r[i], r[i + 1], r[i + 2], r[i + 3]);
+            a[2] = a[2] ^ slice_add4(a[0], a[1], r[0], r[1], r[2], r[3]);
+        } else if (role == SQ_W2) {
+            slice_add4x(a[1], a[2], r[0], r[1], r[2], r[3]);
+        } else if (role == SQ_W4) {
+            a[2] = a[2] ^ r[0] ^ r[1];
+            a[2] = a[2] ^ r[2] ^ r[3];
         } else {  // SQ_N9
             n9 = true;
 #pragma unroll
@@ -273,9 +306,9 @@ __device__ __forceinline__ void slice_task(const uint8_t *chunk, const SliceTerm
                 W2 yb = ~(r[i] | r[i + 1]), zb = r[i] & r[i + 1];
 #pragma unroll
                 for (int b = 0; b < 4; ++b) {
-                    const W2 ty = a[4 + b] & yb, tz = a[8 + b] & zb;
-                    a[4 + b] = a[4 + b] ^ yb;
-                    a[8 + b] = a[8 + b] ^ zb;
+                    const W2 ty = y[b] & yb, tz = z[b] & zb;
+                    y[b] = y[b] ^ yb;
+                    z[b] = z[b] ^ zb;
                     yb = ty;
                     zb = tz;
                 }
@@ -284,49 +317,39 @@ __device__ __forceinline__ void slice_task(const uint8_t *chunk, const SliceTerm
     }
     n9 = __any_sync(~0u, n9);
     for (int o = ln.L; o < 32; o <<= 1) {
-        if (x_half) {
-            a[7] = a[7] ^ slice_shfl(a[7], o);
-            slice_add<0, 7>(a, o);
-        } else {
-            a[3] = a[3] | slice_shfl(a[3], o);
-            slice_add<0, 3>(a, o);
-            if (n9) {
-                slice_add<4, 8>(a, o);
-                slice_add<8, 12>(a, o);
-            }
+        slice_add<0, 3>(a, o);
+        if (n9) {
+            slice_add<0, 4>(y, o);
+            slice_add<0, 4>(z, o);
         }
     }
-    uint8_t *out = planes + ((int)d.plane + (x_half ? 0 : 1)) * plane_bytes;
+    uint8_t *out = planes + ((int)d.plane + 1) * plane_bytes;
     const bool even = d.flags & ST_EVEN, wide = d.flags & ST_WIDE;
     slice_finish(ln, [&](int h, int word) {
-        uint32_t p[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) p[i] = slice_pick(a[i], h);
-        if (!x_half) {
-            const uint32_t k0 = p[0], k1 = p[1], k2 = p[2], kill = p[3];
-            const uint32_t y0 = p[4], y1 = p[5], y2 = p[6], z0 = slice_pick(a[8], h), z1 = slice_pick(a[9], h),
-                           z2 = slice_pick(a[10], h);
-            if (wide) {
-                uint32_t w[8] = {y0, y1, y2, p[7], z0, z1, z2, slice_pick(a[11], h)};
-                slice_store(w, out + plane_bytes + 32 * word);
-            }
-            // class e (e + 1) / 2 + z, e = y + z <= 4 (ST_WIDE: 0)
-            const uint32_t on = wide ? 0u : ~0u;
-            const uint32_t e0 = y0 ^ z0, c0 = y0 & z0, e1 = y1 ^ z1 ^ c0;
-            const uint32_t e2 = (y2 | z2 | (y1 & z1) | (y1 & c0) | (z1 & c0)) & on;
-            const uint32_t t0 = (e0 ^ e1) & on, t1 = (e1 | e2) & on, t2 = e0 & e1 & on;  // e (e + 1) / 2; its bit 3 is e2
-            const uint32_t w0 = z0 & on, w1 = z1 & on, w2 = z2 & on;
-            const uint32_t q0 = t0 & w0, q1 = (t1 & w1) | (t1 & q0) | (w1 & q0), q2 = (t2 & w2) | (t2 & q1) | (w2 & q1);
-            const uint32_t cl0 = t0 ^ w0, cl1 = t1 ^ w1 ^ q0, cl2 = t2 ^ w2 ^ q1, cl3 = e2 ^ q2;
-            p[0] = k1;
-            p[1] = even ? cl0 : k0;
-            p[2] = even ? cl1 : cl0;
-            p[3] = even ? cl2 : cl1;
-            p[4] = even ? cl3 : cl2;
-            p[5] = even ? 0u : cl3;
-            p[6] = kill;
-            p[7] = k2;
+        const uint32_t k0 = slice_pick(a[0], h), k1 = slice_pick(a[1], h), k2 = slice_pick(a[2], h);
+        const uint32_t y0 = slice_pick(y[0], h), y1 = slice_pick(y[1], h), y2 = slice_pick(y[2], h),
+                       z0 = slice_pick(z[0], h), z1 = slice_pick(z[1], h), z2 = slice_pick(z[2], h);
+        if (wide) {
+            uint32_t w[8] = {y0, y1, y2, slice_pick(y[3], h), z0, z1, z2, slice_pick(z[3], h)};
+            slice_store(w, out + plane_bytes + 32 * word);
         }
+        // class e (e + 1) / 2 + z, e = y + z <= 4 (ST_WIDE: 0)
+        const uint32_t on = wide ? 0u : ~0u;
+        const uint32_t e0 = y0 ^ z0, c0 = y0 & z0, e1 = y1 ^ z1 ^ c0;
+        const uint32_t e2 = (y2 | z2 | (y1 & z1) | (y1 & c0) | (z1 & c0)) & on;
+        const uint32_t t0 = (e0 ^ e1) & on, t1 = (e1 | e2) & on, t2 = e0 & e1 & on;  // e (e + 1) / 2; its bit 3 is e2
+        const uint32_t w0 = z0 & on, w1 = z1 & on, w2 = z2 & on;
+        const uint32_t q0 = t0 & w0, q1 = (t1 & w1) | (t1 & q0) | (w1 & q0), q2 = (t2 & w2) | (t2 & q1) | (w2 & q1);
+        const uint32_t cl0 = t0 ^ w0, cl1 = t1 ^ w1 ^ q0, cl2 = t2 ^ w2 ^ q1, cl3 = e2 ^ q2;
+        uint32_t p[8];
+        p[0] = k1;
+        p[1] = even ? cl0 : k0;
+        p[2] = even ? cl1 : cl0;
+        p[3] = even ? cl2 : cl1;
+        p[4] = even ? cl3 : cl2;
+        p[5] = even ? 0u : cl3;
+        p[6] = 0u;
+        p[7] = k2;
         slice_store(p, out + 32 * word);
     });
 }
@@ -558,7 +581,8 @@ __device__ __forceinline__ bool slice_tile(const SampleJob &j, const int64_t s0,
 
         // rows pass: one half term a warp
         for (int task = tid >> 5; task < 2 * nt; task += nthr >> 5)
-                slice_task(chunk, terms[task < nt ? task : task - nt], task >= nt, planes, plane_bytes, ln);
+            if (task < nt) slice_k(chunk, terms[task], planes, plane_bytes, ln);
+            else slice_x(chunk, terms[task - nt], planes, plane_bytes, ln);
         if (__syncthreads_or(!ok)) {
             if (tid == 0) {
                 atomicOr(j.status, (uint32_t)KSIM_FLAG_WAIT_TIMEOUT);
@@ -578,11 +602,11 @@ __device__ __forceinline__ bool slice_tile(const SampleJob &j, const int64_t s0,
                     constexpr int N = S == 1 ? 1 : 4;
                     const uint8_t *pl = planes + (int)T.plane * plane_bytes + byte0 + 16 * h;
                     const uint32_t xw = slice_plane<N>(pl), kw = slice_plane<N>(pl + plane_bytes);
-                    const uint32_t xm = xw & 0x7F7F7F7Fu, km = kw & 0x3F3F3F3Fu;
+                    const uint32_t xm = xw & 0x7F7F7F7Fu, km = kw & 0x7F7F7F7Fu;
                     const uint32_t base = fl & ST_BIG ? 0u : tw;
                     uint32_t at[N];
 #pragma unroll
-                    for (int k = 0; k < N; ++k) at[k] = byte_of(xm, k) * xs + (byte_of(km, k) * 8u + base);
+                    for (int k = 0; k < N; ++k) at[k] = __dp4a(km, 8u << (8 * k), byte_of(xm, k) * xs + base);
                     if (fl & ST_WIDE) {
                         const uint32_t cw = slice_plane<N>(pl + 2 * plane_bytes);
                         const uint8_t *lut = chunk + 16 * (int)T.lut_off16;
@@ -595,7 +619,7 @@ __device__ __forceinline__ bool slice_tile(const SampleJob &j, const int64_t s0,
                     if (fl & ST_BIG) {
 #pragma unroll
                         for (int k = 0; k < N; ++k) {
-                            const uint8_t *p = kw & (0x40u << (8 * k)) ? j.image : j.image + 16 * (size_t)tw + at[k];
+                            const uint8_t *p = j.image + 16 * (size_t)tw + at[k];
                             const uint8_t *q = (const uint8_t *)((uintptr_t)p ^ 8u);
                             a[k] = CG ? __ldcg((const double *)p) : __ldg((const double *)p);
                             b[k] = CG ? __ldcg((const double *)q) : __ldg((const double *)q);
@@ -603,9 +627,8 @@ __device__ __forceinline__ bool slice_tile(const SampleJob &j, const int64_t s0,
                     } else {
 #pragma unroll
                         for (int k = 0; k < N; ++k) {
-                            const uint32_t o = kw & (0x40u << (8 * k)) ? 0u : at[k];
-                            a[k] = *(const double *)(chunk + o);
-                            b[k] = *(const double *)(chunk + (o ^ 8u));
+                            a[k] = *(const double *)(chunk + at[k]);
+                            b[k] = *(const double *)(chunk + (at[k] ^ 8u));
                         }
                     }
                     // times i^(K1 + 2 (K2 ^ S)): the signs go to bit 63

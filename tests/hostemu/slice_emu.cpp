@@ -1,7 +1,7 @@
 // slice_emu.cpp — TEST INFRASTRUCTURE ONLY.
 //
 // Walks a component's sliced stream (ksim_b200/csrc/slice.cpp) on the CPU,
-// one parameter row at a time with the roles the kernel gives each quad, so
+// one parameter row at a time with the roles the kernel gives each group, so
 // the tests can check the stream against the oracle without a GPU.
 #include <cstdint>
 #include <cstring>
@@ -77,7 +77,7 @@ int slice_emu_eval(const ksim_graph_desc *g, int n, int F, int gi, const uint8_t
                 std::memcpy(&d, base + SLICE_HEAD + t * sizeof(SliceTerm), sizeof(d));
                 const uint8_t *list = base + 16 * d.list_off16;
                 int r[8], kill = 0, K = 0, y = 0, z = 0, X = 0, S = 0;
-                for (int q = 0; q < d.n_k + d.n_x; ++q) {
+                for (int q = 0; q < d.n_k + d.n_x1 + d.n_x0 + d.n_xp; ++q) {
                         uint32_t entry;
                         std::memcpy(&entry, list + 4 * q, 4);
                         const int m = SLICE_GROUP, role = (int)(entry >> 24 & 15u);
@@ -100,12 +100,11 @@ int slice_emu_eval(const ksim_graph_desc *g, int n, int F, int gi, const uint8_t
                         default: X += sum; break;
                         }
                     }
-                if (kill) continue;
                 K = (K + 4 * S) & 7;
                 const int e = y + z;
                 const int cls = (d.flags & ST_WIDE) ? base[16 * d.lut_off16 + (y | z << 4)] : e * (e + 1) / 2 + z;
                 const int col = (d.flags & ST_EVEN) ? cls : 2 * cls + (K & 1);
-                const size_t at = (size_t)X * d.xs + (size_t)col * 16;
+                const size_t at = (size_t)(kill ? 0 : X + 1) * d.xs + (size_t)col * 16;
                 const uint8_t *tab = (d.flags & ST_BIG) ? s.bytes.data() + 16 * (size_t)d.tab : base + d.tab;
                 double re, im;
                 std::memcpy(&re, tab + at, 8);

@@ -108,7 +108,7 @@ def test_phase_pair_classes(emu, oracle_port):
 
 def test_not_sliced(emu):
     """Terms without a proof (int64 may wrap; scales beyond the normal range),
-    more than 127 lambda rows, more than 254 parameters."""
+    more than 126 lambda rows, more than 254 parameters."""
     rng = np.random.default_rng(3)
     wrap = synth.random_graph(rng, 1, 10, 250, 0, 0, 0)
     wrap.np_phases[:], wrap.np_counts[:] = 1, 250
@@ -119,5 +119,5 @@ def test_not_sliced(emu):
     assert info(emu, [synth.random_graph(rng, 1, 254, 4, 1, 1, 1)], 254)["ok"]
     assert not info(emu, [synth.random_graph(rng, 1, 255, 4, 1, 1, 1)], 255)["ok"]
     empty = synth.random_graph(rng, 0, 10, 4, 1, 1, 1)
-    assert info(emu, [empty], 10) == {"ok": 1, "rows": 10, "planes": 0, "chunks": 1, "bytes": 32, "terms": 0,
+    assert info(emu, [empty], 10) == {"ok": 1, "rows": 10, "planes": 0, "chunks": 1, "bytes": 16, "terms": 0,
                                       "wide": 0, "big": 0}
