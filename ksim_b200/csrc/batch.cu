@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(256, 2) k_batch_s(const __grid_constant__ PT P
     __shared__ int s_item;
     uint8_t *ring = smem + P.slot_bytes;
     uint64_t *bar = (uint64_t *)ring;
-    ring_init(bar);
+    slice_ring_init(bar);
     pdl_launch_dependents();
     uint32_t g = 0;
     for (;;) {
@@ -454,7 +454,7 @@ ksim_status ksim_batch_create(const ksim_batch_job *jobs, int32_t n_jobs, const 
         BatchClass &k = b->cls[c];
         if (items[c].empty()) continue;
         if (k.sliced) k.threads = 256;
-        k.smem = k.sliced ? (size_t)k.ring_off + BAR_BYTES + NSLOT * SLICE_SLOT
+        k.smem = k.sliced ? (size_t)k.ring_off + BAR_BYTES + SLICE_RING
                           : batch_smem_bytes(k.slot, k.max_w, k.threads);
         std::vector<int> order(items[c].size());
         std::iota(order.begin(), order.end(), 0);

@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(THREADS, CTAS) k_slice(const SampleJob j, cons
     extern __shared__ __align__(128) uint8_t smem[];
     uint8_t *ring = smem + slice_ring_off(j.s_rows, j.s_planes, shots);
     uint64_t *bar = (uint64_t *)ring;
-    ring_init(bar);
+    slice_ring_init(bar);
     uint32_t g = 0;
     const int64_t s0 = (int64_t)blockIdx.x * tile;
     slice_tile<S, false, EVAL>(j, s0, s0 + tile < j.B ? s0 + tile : j.B, shots, smem, slice_rows_bytes(j.s_rows, shots), bar,

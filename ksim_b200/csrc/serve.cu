@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(SERVE_THREADS, 2) k_serve(ServeJob *jobs, Serv
     __shared__ __align__(16) SampleJob s_job;
     __shared__ int s_slot, s_tile, s_shots;
     uint64_t *bar = (uint64_t *)(smem + SERVE_RING);
-    ring_init(bar);
+    slice_ring_init(bar);
     uint32_t g = 0;
     const long long t_start = global_ns();
     unsigned backoff = 64;

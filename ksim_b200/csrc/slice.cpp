@@ -264,6 +264,7 @@ std::vector<Group> make_groups(const std::vector<Row> &rows, int step, const Row
 
 struct TermOutBytes {
     SliceTerm d;
+    SliceValue v;
     std::vector<Group> groups;  // role by role
     size_t rows_bytes() const
     {
@@ -371,6 +372,7 @@ bool build_term(const ksim_graph_desc &g, int t, int zero_row, TermOutBytes &o)
 
     SliceTerm &d = o.d;
     std::memset(&d, 0, sizeof(d));
+    std::memset(&o.v, 0, sizeof(o.v));
     d.flags = (uint16_t)((wide ? ST_WIDE : 0u) | (even ? ST_EVEN : 0u));
     o.planes = wide ? 3 : 2;
     std::vector<Group> role[SQ_ROLES];
@@ -416,7 +418,7 @@ bool build_term(const ksim_graph_desc &g, int t, int zero_row, TermOutBytes &o)
     }
     const int n_par = even ? 1 : 2;
     const size_t xs = cls.size() * (size_t)n_par * 16;
-    d.xs = (uint16_t)xs;
+    o.v.xs = (uint16_t)xs;
     o.tab.assign(xs * (size_t)(nx + 2), 0);
 
     base.e += R.n_two;
@@ -492,23 +494,25 @@ void build_slices(const ksim_graph_desc *gs, const HostImage &img, SliceImage &o
         const ksim_graph_desc &g = gs[k];
         int t = 0;
         do {
-            // the terms of this chunk: as many as fit the slot and the planes
+            // the terms of this chunk: as many as fit the slots and the planes
             std::vector<TermOutBytes> terms;
-            size_t bytes = SLICE_HEAD;
+            size_t rows_bytes = SLICE_HEAD, tab_bytes = 0;
             int planes = 0;
             for (; t < g.G; ++t) {
                 TermOutBytes o;
                 if (!build_term(g, t, rows, o)) return;
                 const bool is_big = o.tab.size() > (size_t)SLICE_BIG_TABLE;
                 if (is_big) o.d.flags |= ST_BIG;
-                const size_t need = sizeof(SliceTerm) + o.rows_bytes() + o.lut.size() +
-                                    (is_big ? 0 : o.tab.size());
-                if (SLICE_HEAD + need > (size_t)SLICE_SLOT) return;
-                if (bytes + need > (size_t)SLICE_SLOT || planes + o.planes > SLICE_MAX_PLANES ||
-                    terms.size() == (size_t)SLICE_MAX_TERMS)
+                const size_t need_r = sizeof(SliceTerm) + o.rows_bytes();
+                const size_t need_t = sizeof(SliceValue) + o.lut.size() + (is_big ? 0 : o.tab.size());
+                if (SLICE_HEAD + need_r > (size_t)SLICE_SLOT) return;
+                if (rows_bytes + need_r > (size_t)SLICE_SLOT || tab_bytes + need_t > (size_t)SLICE_TABLES ||
+                    planes + o.planes > SLICE_MAX_PLANES || terms.size() == (size_t)SLICE_MAX_TERMS)
                     break;
-                o.d.plane = (uint16_t)planes;
-                bytes += need;
+                o.d.plane = o.v.plane = (uint16_t)planes;
+                o.v.flags = o.d.flags;
+                rows_bytes += need_r;
+                tab_bytes += need_t;
                 planes += o.planes;
                 terms.push_back(std::move(o));
             }
@@ -518,7 +522,8 @@ void build_slices(const ksim_graph_desc *gs, const HostImage &img, SliceImage &o
             c.n_terms = (int32_t)terms.size();
             c.end_of_graph = t >= g.G ? 1 : 0;
             std::vector<uint8_t> body(SLICE_HEAD + sizeof(SliceTerm) * terms.size(), 0);
-            for (TermOutBytes &o : terms) {
+            for (size_t i = 0; i < terms.size(); ++i) {
+                TermOutBytes &o = terms[i];
                 o.d.list_off16 = (uint16_t)(body.size() / 16);
                 size_t at = body.size() + (4 * o.groups.size() + 15) / 16 * 16;
                 for (const Group &x : o.groups) {
@@ -528,22 +533,27 @@ void build_slices(const ksim_graph_desc *gs, const HostImage &img, SliceImage &o
                 }
                 pad(body, 16);
                 for (const Group &x : o.groups) body.insert(body.end(), x.bytes.begin(), x.bytes.end());
-                o.d.lut_off16 = (uint16_t)(body.size() / 16);
-                body.insert(body.end(), o.lut.begin(), o.lut.end());
-            }
-            for (size_t i = 0; i < terms.size(); ++i) {
-                TermOutBytes &o = terms[i];
-                if (o.d.flags & ST_BIG) {
-                    refs.push_back({(size_t)c.off + SLICE_HEAD + i * sizeof(SliceTerm), big.size()});
-                    big.insert(big.end(), o.tab.begin(), o.tab.end());
-                } else {
-                    o.d.tab = (uint32_t)body.size();
-                    body.insert(body.end(), o.tab.begin(), o.tab.end());
-                }
                 std::memcpy(&body[SLICE_HEAD + i * sizeof(SliceTerm)], &o.d, sizeof(SliceTerm));
             }
             c.bytes = (int32_t)body.size();
+            // (never empty: a copy is at least 16 bytes)
+            std::vector<uint8_t> tabs(sizeof(SliceValue) * std::max<size_t>(1, terms.size()), 0);
+            for (size_t i = 0; i < terms.size(); ++i) {
+                TermOutBytes &o = terms[i];
+                o.v.lut_off16 = (uint16_t)(tabs.size() / 16);
+                tabs.insert(tabs.end(), o.lut.begin(), o.lut.end());
+                if (o.d.flags & ST_BIG) {
+                    refs.push_back({(size_t)c.off + body.size() + i * sizeof(SliceValue), big.size()});
+                    big.insert(big.end(), o.tab.begin(), o.tab.end());
+                } else {
+                    o.v.tab = (uint32_t)tabs.size();
+                    tabs.insert(tabs.end(), o.tab.begin(), o.tab.end());
+                }
+                std::memcpy(&tabs[i * sizeof(SliceValue)], &o.v, sizeof(SliceValue));
+            }
+            c.pad0 = (int32_t)tabs.size();
             out.bytes.insert(out.bytes.end(), body.begin(), body.end());
+            out.bytes.insert(out.bytes.end(), tabs.begin(), tabs.end());
             out.max_planes = std::max(out.max_planes, planes);
             out.chunks.push_back(c);
         } while (t < g.G);
@@ -559,13 +569,18 @@ void build_slices(const ksim_graph_desc *gs, const HostImage &img, SliceImage &o
             h.ahead_bytes = (uint32_t)a.bytes;
             h.ahead_off16 = (uint32_t)(a.off / 16);
         }
+        if (i + 1 < out.chunks.size()) {
+            const ChunkDir &a = out.chunks[i + 1];
+            h.tab_bytes = (uint32_t)a.pad0;
+            h.tab_off16 = (uint32_t)((a.off + a.bytes) / 16);
+        }
         std::memcpy(&out.bytes[(size_t)c.off], &h, sizeof(h));
     }
     pad(out.bytes, 16);
     const size_t at = out.bytes.size();
     for (const BigRef &r : refs) {
         const uint32_t off = (uint32_t)((at + r.off) / 16);
-        std::memcpy(&out.bytes[r.desc + offsetof(SliceTerm, tab)], &off, 4);
+        std::memcpy(&out.bytes[r.desc + offsetof(SliceValue, tab)], &off, 4);
     }
     out.bytes.insert(out.bytes.end(), big.begin(), big.end());
     if (out.bytes.empty()) out.bytes.resize(16, 0);

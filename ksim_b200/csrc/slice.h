@@ -45,19 +45,24 @@ namespace ksim {
 // slots are bytes, so at most 255 rows.
 constexpr int SLICE_ROW = 128;
 constexpr int SLICE_MAX_ROWS = 254;   // parameters; one more row is all zero
-constexpr int SLICE_SLOT = 24576;     // bytes of a staged chunk
+constexpr int SLICE_SLOT = 8192;      // bytes of a staged chunk's rows (two slots)
+constexpr int SLICE_TABLES = 32768;   // bytes of its tables (one slot)
 constexpr int SLICE_MAX_PLANES = 16;  // result bytes per shot of a chunk's terms
 constexpr int SLICE_MAX_TERMS = 8;    // of a chunk
 constexpr int SLICE_AHEAD = 2;        // chunks staged at once
 
-// A chunk starts with what a CTA needs to know of it and of the chunk
-// SLICE_AHEAD behind it.
+// A chunk has two parts, staged by copies of their own: the rows (this head,
+// its terms' SliceTerm, group lists and groups) and, behind them, the tables
+// (SliceValue, then look-up tables and value tables).  The head says what a
+// CTA needs to know of the chunk, of the next one's tables and of the rows of
+// the chunk SLICE_AHEAD behind it.
 struct SliceChunk {
     uint16_t n_terms, end_of_graph;
-    uint32_t graph, ahead_bytes, ahead_off16;
+    uint32_t graph, ahead_bytes, ahead_off16, tab_bytes, tab_off16;
+    uint32_t pad[2];
 };
 constexpr int SLICE_HEAD = sizeof(SliceChunk);
-static_assert(SLICE_HEAD == 16, "SliceChunk layout");
+static_assert(SLICE_HEAD == 32, "SliceChunk layout");
 constexpr int SLICE_BIG_TABLE = 16384;  // larger tables stay in global memory
 
 enum : uint32_t { ST_WIDE = 1u, ST_BIG = 2u, ST_EVEN = 4u };
@@ -78,30 +83,35 @@ enum : uint32_t { ST_WIDE = 1u, ST_BIG = 2u, ST_EVEN = 4u };
 // pairs, into S; kill.
 enum { SQ_W1, SQ_W2, SQ_W4, SQ_N9, SQ_PPK, SQ_X1, SQ_X0, SQ_PPX, SQ_KILL, SQ_ROLES };
 
-// One term of a chunk, behind its head.  Its rows come in groups of
-// four, listed role by role as u32: bits 0-15 the group's offset in the chunk /
+// One term of a chunk, in either part.  Its rows come in groups of four, listed role by role as u32: bits 0-15 the group's offset in the chunk /
 // 16, 16-23 its index slots a row, 24-27 the role.
 constexpr int SLICE_GROUP = 4;
 struct SliceTerm {
-    uint32_t tab;         // byte offset of the table in the chunk (ST_BIG: / 16, in the image)
-    uint16_t xs;          // table bytes per X step
-    uint16_t flags;
-    uint16_t list_off16;  // group list (16-byte units, in the chunk)
-    uint16_t lut_off16;   // ST_WIDE: 256 bytes, class of y | z << 4
+    uint16_t list_off16;  // group list (16-byte units, in the rows part)
     uint16_t plane;       // first result plane
+    uint16_t flags;
     uint16_t n_k;         // groups of the K half
     uint16_t n_x1, n_x0;  // of X with and without S,
     uint16_t n_xp;        // of the X half's pairs and kill rows
-    uint16_t pad[5];
+    uint16_t pad;
 };
-static_assert(sizeof(SliceTerm) == 32, "SliceTerm layout");
+static_assert(sizeof(SliceTerm) == 16, "SliceTerm layout");
+struct SliceValue {
+    uint32_t tab;        // byte offset of the table in the tables part (ST_BIG: / 16, in the image)
+    uint16_t xs;         // table bytes per X step
+    uint16_t flags;
+    uint16_t lut_off16;  // ST_WIDE: 256 bytes, class of y | z << 4
+    uint16_t plane;
+    uint32_t pad;
+};
+static_assert(sizeof(SliceValue) == 16, "SliceValue layout");
 
 struct SliceImage {
     bool ok = false;
     int rows = 0;        // parameter rows
     int max_planes = 0;  // of any chunk
     std::vector<uint8_t> bytes;
-    std::vector<ChunkDir> chunks;  // offsets in bytes
+    std::vector<ChunkDir> chunks;  // off, bytes: the rows part; pad0: bytes of the tables behind it
 };
 
 // Build the sliced stream of a component whose image is `img` (build_image on

@@ -5,24 +5,37 @@
 // runs two passes:
 //   rows    a warp takes one half of a term (its K roles or its X roles): L
 //           lanes cover the tile's shots, 64 each, and the 32 / L lane groups
-//           share the groups of four rows of every role.  A lane forms parity rows as XORs
-//           of a few parameter words and adds them into bit-sliced counters
-//           (carry-save adders); the groups' counters are added over
-//           shuffles, and the eight result planes become one byte per shot by
-//           in-register 8 x 8 bit transposes;
+//           share the groups of four rows of every role.  A lane forms parity
+//           rows as XORs of a few parameter words and adds them into
+//           bit-sliced counters (carry-save adders); the lane groups' counters
+//           are added over shuffles, and the eight result planes become one
+//           byte per shot by in-register 8 x 8 bit transposes;
 //   values  a thread takes its S shots: two result bytes a term give the
-//           table entry (a complex double), its rotation by i^k and whether
-//           the term is dead; the entries are added in term order.
+//           table entry (a complex double) and its rotation by i^k; the
+//           entries are added in term order.
 // At a graph's end each thread makes its Bernoulli draws and the warp writes
 // the sampled output's row with ballots (kokkos_sim.cpp:214-230).
 //
-// Chunks are staged by TMA bulk copies in a two-slot ring as in
-// sample_tile.cuh, with the same bounded waits.
+// Chunks are staged by TMA bulk copies with bounded waits, the rows of a chunk
+// in a ring of two slots, its tables in one slot: the tables' copy is issued
+// when the chunk before is done and hides behind the rows pass, which needs
+// only the rows.  One 24 KB slot for both held 3 terms on average where a
+// term's table is 5 KB (6 of 16 warps had a half term); apart, chunks have 5 to
+// 8 terms: 3,001 shots of such a program 0.332 -> 0.248 ms, of the 40-output
+// program 0.219 -> 0.191.
+//
+// What bounds it: issued instructions and their latency (four warps a
+// scheduler, 54 % of the issue slots, the ALU pipe 47 % busy, shared memory
+// 45 %, HBM idle).  Of ~5,100 warp instructions a term and 2,048 shots the
+// rows take ~2,400, the values ~1,700, the draws ~900.
 #pragma once
 #include "sample_tile.cuh"
 #include "slice.h"
 
 namespace ksim {
+
+// The ring: NSLOT slots of rows, one of tables, a barrier each.
+constexpr int SLICE_RING = NSLOT * SLICE_SLOT + SLICE_TABLES;
 
 // Shared memory of a sliced tile of `shots` (64 to 2,048, a power of two):
 // parameter rows, result planes, then the barriers and the ring.
@@ -38,7 +51,7 @@ __host__ __device__ constexpr int slice_ring_off(int rows, int planes, int shots
 }
 __host__ __device__ constexpr int slice_smem_bytes(int rows, int planes, int shots)
 {
-    return slice_ring_off(rows, planes, shots) + BAR_BYTES + NSLOT * SLICE_SLOT;
+    return slice_ring_off(rows, planes, shots) + BAR_BYTES + SLICE_RING;
 }
 
 // The most a sliced CTA takes (254 parameters, 2,048 shots): every sliced
@@ -61,8 +74,10 @@ __device__ __forceinline__ W2 maj(W2 x, W2 y, W2 z)
 
 // The four rows of a group for this lane's 64 shots.  lane8: the shared
 // address of the lane's column of the parameter rows.  A slot's address is one
-// dot product (byte k of the word times the row pitch, plus the column).  Most
-// rows have one to four parameters: a straight path each.
+// dot product (byte k of the word times the row pitch, plus the column); slots
+// beyond a row's parameters name the zero row.  ONE: the warp has one lane
+// group, so its lanes take the same path, and the common lengths have one
+// each; else the lanes of several groups run two slots at a time together.
 __device__ __forceinline__ W2 slice_ld(uint32_t x, int k, uint32_t lane8)
 {
     W2 v;
@@ -70,55 +85,34 @@ __device__ __forceinline__ W2 slice_ld(uint32_t x, int k, uint32_t lane8)
                  : "r"(__dp4a(x, (uint32_t)SLICE_ROW << (8 * k), lane8)));
     return v;
 }
+__device__ __forceinline__ void slice_two(const uint4 &u, int k, uint32_t lane8, W2 (&r)[SLICE_GROUP])
+{
+    const uint32_t v[4] = {u.x, u.y, u.z, u.w};
+    W2 x[4], y[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[i] = slice_ld(v[i], k, lane8);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) y[i] = slice_ld(v[i], k + 1, lane8);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r[i] = r[i] ^ x[i] ^ y[i];
+}
 __device__ __forceinline__ void slice_rows(uint32_t entry, const uint8_t *chunk, uint32_t lane8, W2 (&r)[SLICE_GROUP])
 {
     const uint4 *p = (const uint4 *)(chunk + 16u * (entry & 0xFFFFu));
     int n = (int)((entry >> 16) & 0xFFu);
-    const uint4 inv4 = p[0], u4 = p[1];
-    const uint32_t inv[4] = {inv4.x, inv4.y, inv4.z, inv4.w};
-    const uint32_t u[4] = {u4.x, u4.y, u4.z, u4.w};
-    if (n == 1) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) r[i] = slice_ld(u[i], 0, lane8);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) r[i] = {r[i].a ^ inv[i], r[i].b ^ inv[i]};
-        return;
-    }
-    {
-        W2 x[4], y[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) x[i] = slice_ld(u[i], 0, lane8);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) y[i] = slice_ld(u[i], 1, lane8);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) r[i] = {x[i].a ^ y[i].a ^ inv[i], x[i].b ^ y[i].b ^ inv[i]};
-    }
-    if (n == 2) return;
-    if (n == 3) {
-        W2 x[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) x[i] = slice_ld(u[i], 2, lane8);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) r[i] = r[i] ^ x[i];
-        return;
-    }
-    auto pair = [&](const uint32_t (&v)[4], int k) {
-        W2 x[4], y[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) x[i] = slice_ld(v[i], k, lane8);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) y[i] = slice_ld(v[i], k + 1, lane8);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) r[i] = r[i] ^ x[i] ^ y[i];
-    };
-    pair(u, 2);
-    for (n -= 4, p += 2; n > 0; n -= 2) {  // (unused slots name the zero row)
-        const uint4 v4 = *p;
-        const uint32_t v[4] = {v4.x, v4.y, v4.z, v4.w};
-        pair(v, 0);
-        if ((n -= 2) <= 0) break;
-        pair(v, 2);
-        ++p;
+    const uint4 inv = p[0], u = p[1];
+    r[0] = {inv.x, inv.x};
+    r[1] = {inv.y, inv.y};
+    r[2] = {inv.z, inv.z};
+    r[3] = {inv.w, inv.w};
+    slice_two(u, 0, lane8, r);
+    if (n <= 2) return;
+    slice_two(u, 2, lane8, r);
+    for (n -= 4, p += 2; n > 0; n -= 4, ++p) {
+        const uint4 v = *p;
+        slice_two(v, 0, lane8, r);
+        if (n <= 2) break;
+        slice_two(v, 2, lane8, r);
     }
 }
 
@@ -177,15 +171,14 @@ struct SliceLane {
     int L, li, grp, n_grp;
     uint32_t lane8;
 };
-template <typename F>
+template <bool ONE, typename F>
 __device__ __forceinline__ void slice_finish(const SliceLane &ln, F &&store)
 {
-    if (ln.grp > 1) return;
-    int h = ln.grp;
-    for (;;) {
-        store(h, ln.li + h * ln.L);
-        if (ln.n_grp > 1 || h) break;
-        h = 1;
+    if (ONE) {
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) store(h, ln.li + 32 * h);
+    } else if (ln.grp < 2) {
+        store(ln.grp, ln.li + ln.grp * ln.L);
     }
 }
 __device__ __forceinline__ uint32_t slice_pick(W2 x, int h) { return h ? x.b : x.a; }
@@ -216,36 +209,32 @@ __device__ __forceinline__ void slice_add4x(W2 &x0, W2 &x1, W2 b0, W2 b1, W2 b2,
 // a look at the role: of ~3,200 warp instructions a term's rows pass took for
 // 2,048 shots, ~700 were the one loop's role dispatch and ~450 register moves
 // (606,208 shots of the 40-output program: 0.783 -> 0.711 ms).
+template <bool ONE>
 __device__ __forceinline__ void slice_x(const uint8_t *chunk, const SliceTerm &d, uint8_t *planes, int plane_bytes,
                                         const SliceLane &ln)
 {
     const uint32_t *list = (const uint32_t *)(chunk + 16 * (int)d.list_off16) + (int)d.n_k;
-    const uint32_t one = ln.grp == 0 ? ~0u : 0u;
-    W2 a[8], kill = {0u, 0u}, s = {0u, 0u};
+    const int n_x = d.n_x1 + d.n_x0, n = n_x + d.n_xp, n_x1 = d.n_x1, step = ONE ? 1 : ln.n_grp;
+    const uint32_t one = ONE || ln.grp == 0 ? ~0u : 0u;
+    W2 a[7], kill = {0u, 0u}, s = {one, one};
     a[0] = {one, one};
 #pragma unroll
-    for (int i = 1; i < 8; ++i) a[i] = {0u, 0u};
-    int q = ln.grp, n = d.n_x1;
-    for (int phase = 0; phase < 2; ++phase) {
-        for (; q < n; q += ln.n_grp) {
-            W2 r[SLICE_GROUP];
-            slice_rows(list[q], chunk, ln.lane8, r);
-            W2 c = slice_add4(a[0], a[1], r[0], r[1], r[2], r[3]);
+    for (int i = 1; i < 7; ++i) a[i] = {0u, 0u};
+    int q = ONE ? 0 : ln.grp;
+    for (; q < n_x; q += step) {
+        W2 r[SLICE_GROUP];
+        slice_rows(list[q], chunk, ln.lane8, r);
+        W2 c = slice_add4(a[0], a[1], r[0], r[1], r[2], r[3]);
 #pragma unroll
-            for (int i = 2; i < 7; ++i) {
-                const W2 t = a[i] & c;
-                a[i] = a[i] ^ c;
-                c = t;
-            }
+        for (int i = 2; i < 7; ++i) {
+            const W2 t = a[i] & c;
+            a[i] = a[i] ^ c;
+            c = t;
         }
-        if (phase == 0) {
-            s = a[0];  // the parity so far, complemented by `one`
-            n += d.n_x0;
-        }
+        if (q < n_x1) s = a[0];  // the parity so far, complemented by `one`
     }
     s = {s.a ^ one, s.b ^ one};
-    n += d.n_xp;
-    for (; q < n; q += ln.n_grp) {
+    for (; q < n; q += step) {
         const uint32_t e = list[q];
         W2 r[SLICE_GROUP];
         slice_rows(e, chunk, ln.lane8, r);
@@ -257,13 +246,13 @@ __device__ __forceinline__ void slice_x(const uint8_t *chunk, const SliceTerm &d
             kill = kill | r[2] | r[3];
         }
     }
-    for (int o = ln.L; o < 32; o <<= 1) {
+    for (int o = ONE ? 32 : ln.L; o < 32; o <<= 1) {
         s = s ^ slice_shfl(s, o);
         kill = kill | slice_shfl(kill, o);
         slice_add<0, 7>(a, o);
     }
     uint8_t *out = planes + (int)d.plane * plane_bytes;
-    slice_finish(ln, [&](int h, int word) {
+    slice_finish<ONE>(ln, [&](int h, int word) {
         uint32_t p[8];
         const uint32_t live = ~slice_pick(kill, h);
 #pragma unroll
@@ -274,6 +263,7 @@ __device__ __forceinline__ void slice_x(const uint8_t *chunk, const SliceTerm &d
 }
 
 // The K half: planes a[0..2] K, y[] and z[] the p and q counts.
+template <bool ONE>
 __device__ __forceinline__ void slice_k(const uint8_t *chunk, const SliceTerm &d, uint8_t *planes, int plane_bytes,
                                         const SliceLane &ln)
 {
@@ -285,7 +275,7 @@ __device__ __forceinline__ void slice_k(const uint8_t *chunk, const SliceTerm &d
 #pragma unroll
     for (int i = 0; i < 4; ++i) y[i] = z[i] = {0u, 0u};
     bool n9 = false;
-    for (int q = ln.grp; q < n; q += ln.n_grp) {
+    for (int q = ONE ? 0 : ln.grp; q < n; q += ONE ? 1 : ln.n_grp) {
         const uint32_t e = list[q], role = e >> 24;
         W2 r[SLICE_GROUP];
         slice_rows(e, chunk, ln.lane8, r);
@@ -316,7 +306,7 @@ __device__ __forceinline__ void slice_k(const uint8_t *chunk, const SliceTerm &d
         }
     }
     n9 = __any_sync(~0u, n9);
-    for (int o = ln.L; o < 32; o <<= 1) {
+    for (int o = ONE ? 32 : ln.L; o < 32; o <<= 1) {
         slice_add<0, 3>(a, o);
         if (n9) {
             slice_add<0, 4>(y, o);
@@ -325,7 +315,7 @@ __device__ __forceinline__ void slice_k(const uint8_t *chunk, const SliceTerm &d
     }
     uint8_t *out = planes + ((int)d.plane + 1) * plane_bytes;
     const bool even = d.flags & ST_EVEN, wide = d.flags & ST_WIDE;
-    slice_finish(ln, [&](int h, int word) {
+    slice_finish<ONE>(ln, [&](int h, int word) {
         const uint32_t k0 = slice_pick(a[0], h), k1 = slice_pick(a[1], h), k2 = slice_pick(a[2], h);
         const uint32_t y0 = slice_pick(y[0], h), y1 = slice_pick(y[1], h), y2 = slice_pick(y[2], h),
                        z0 = slice_pick(z[0], h), z1 = slice_pick(z[1], h), z2 = slice_pick(z[2], h);
@@ -398,19 +388,65 @@ __device__ __forceinline__ uint32_t byte_of(uint32_t x, int k) { return (x >> (8
 
 // A thread's bytes of a result plane.
 template <int N>
-__device__ __forceinline__ uint32_t slice_plane(const uint8_t *p)
+__device__ __forceinline__ uint32_t slice_plane(uint32_t p)
 {
-    return N == 4 ? *(const uint32_t *)p : *p;
+    uint32_t x;
+    if (N == 4) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(x) : "r"(p));
+    else asm volatile("ld.shared.u8 %0, [%1];" : "=r"(x) : "r"(p));
+    return x;
 }
 
-// Issue the copy of a chunk (`bytes` at `off` of the job's stream) as the
-// gidx-th of the CTA.
+// Issue the copies of a chunk's rows and of its tables (`bytes` at `off` of
+// the job's stream) as the gidx-th of the CTA.
 __device__ __forceinline__ void slice_issue(const SampleJob &j, int64_t off, uint32_t bytes, uint32_t gidx,
                                             uint64_t *bar, uint8_t *slots)
 {
     const int slot = (int)(gidx & (NSLOT - 1));
     mbar_arrive_expect_tx(&bar[slot], bytes);
     tma_bulk_g2s(slots + (size_t)slot * SLICE_SLOT, j.image + off, bytes, &bar[slot]);
+}
+__device__ __forceinline__ void slice_issue_tables(const SampleJob &j, int64_t off, uint32_t bytes, uint64_t *bar,
+                                                   uint8_t *slots)
+{
+    mbar_arrive_expect_tx(&bar[NSLOT], bytes);
+    tma_bulk_g2s(slots + NSLOT * SLICE_SLOT, j.image + off, bytes, &bar[NSLOT]);
+}
+// A chunk's wait, the same for all lanes: usually the copy is there; what
+// follows a first try that ran out is out of line (a job's own bound counts
+// every poll).
+__device__ __forceinline__ bool mbar_try(uint64_t *bar, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok;
+}
+static __device__ __noinline__ bool slice_wait_out(uint64_t *bar, uint32_t parity, long long polls)
+{
+    return polls > 0 ? mbar_poll(bar, parity, polls) : mbar_wait(bar, parity);
+}
+__device__ __forceinline__ bool slice_wait(const SampleJob &j, uint64_t *bar, uint32_t parity)
+{
+    return __all_sync(~0u, (j.wait_limit <= 0 && mbar_try(bar, parity)) ||
+                               slice_wait_out(bar, parity, j.wait_limit));
+}
+// The ring's barriers (once per CTA).
+__device__ __forceinline__ void slice_ring_init(uint64_t *bar)
+{
+    if (threadIdx.x == 0) mbar_init(&bar[NSLOT], 1);
+    ring_init(bar);
+}
+
+__device__ __forceinline__ uint2 lds64(uint32_t a)
+{
+    uint2 x;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(x.x), "=r"(x.y) : "r"(a));
+    return x;
 }
 
 // Sample shots [s0, s_end) of job j in a tile of `shots`, S of them a thread
@@ -421,16 +457,19 @@ __device__ __forceinline__ void slice_issue(const SampleJob &j, int64_t off, uin
 // whole parameter vectors; |A| (EVAL_ABS) or A (EVAL_COMPLEX) goes to j.amp.
 template <int S, bool CG = false, int EVAL = -1>
 __device__ __forceinline__ bool slice_tile(const SampleJob &j, const int64_t s0, const int64_t s_end, int shots,
-                                           uint8_t *smem, int planes_off, uint64_t *bar, uint8_t *slots, uint32_t &g)
+                                           uint8_t *smem, int planes_off, uint64_t *bar, uint8_t *, uint32_t &g)
 {
+    uint8_t *slots = (uint8_t *)bar + BAR_BYTES;
     static_assert(S == 1 || S == 4 || S == 8, "shots per thread");
     const int tid = threadIdx.x, lane = tid & 31, nthr = (int)blockDim.x;
     uint8_t *planes = smem + planes_off;
     const int plane_bytes = shots;
     const int F = j.F, R = j.s_rows;
     const int region = slice_region(R);
+    constexpr bool ONE = S == 8;
+    const int warp = __shfl_sync(~0u, tid >> 5, 0);  // (the same in all lanes, also to the compiler)
     SliceLane ln;
-    ln.L = shots >> 6;
+    ln.L = ONE ? 32 : shots >> 6;
     ln.li = lane & (ln.L - 1);
     ln.grp = lane / ln.L;
     ln.n_grp = 32 / ln.L;
@@ -567,6 +606,7 @@ __device__ __forceinline__ bool slice_tile(const SampleJob &j, const int64_t s0,
         for (int c = 0; c < NSLOT && c < nch; ++c) {
             const ChunkDir d = ld_chunk<CG>(j.cdir + c);
             slice_issue(j, d.off, (uint32_t)d.bytes, g + (uint32_t)c, bar, slots);
+            if (c == 0) slice_issue_tables(j, d.off + d.bytes, (uint32_t)d.pad0, bar, slots);
         }
 
     for (int c = 0; c < nch; ++c) {
@@ -574,72 +614,79 @@ __device__ __forceinline__ bool slice_tile(const SampleJob &j, const int64_t s0,
         const int slot = (int)(gc & (NSLOT - 1));
         const uint8_t *chunk = slots + (size_t)slot * SLICE_SLOT;
         const SliceTerm *terms = (const SliceTerm *)(chunk + SLICE_HEAD);
-        const bool ok = __all_sync(~0u, j.wait_limit > 0 ? mbar_poll(&bar[slot], par, j.wait_limit)
-                                                         : mbar_wait(&bar[slot], par));
+        const bool ok = slice_wait(j, &bar[slot], par);
         const SliceChunk &d = *(const SliceChunk *)chunk;
         const int nt = ok ? d.n_terms : 0;
 
         // rows pass: one half term a warp
-        for (int task = tid >> 5; task < 2 * nt; task += nthr >> 5)
-            if (task < nt) slice_k(chunk, terms[task], planes, plane_bytes, ln);
-            else slice_x(chunk, terms[task - nt], planes, plane_bytes, ln);
-        if (__syncthreads_or(!ok)) {
+        for (int task = warp; task < 2 * nt; task += nthr >> 5)
+            if (task < nt) slice_k<ONE>(chunk, terms[task], planes, plane_bytes, ln);
+            else slice_x<ONE>(chunk, terms[task - nt], planes, plane_bytes, ln);
+        if (__syncthreads_or(!slice_wait(j, &bar[NSLOT], gc & 1u) || !ok)) {
             if (tid == 0) {
                 atomicOr(j.status, (uint32_t)KSIM_FLAG_WAIT_TIMEOUT);
                 mbar_wait(&bar[slot], par);
+                mbar_wait(&bar[NSLOT], gc & 1u);
                 if (c + 1 < nch) mbar_wait(&bar[slot ^ 1], ((gc + 1) / NSLOT) & 1u);
             }
             return false;
         }
 
         // values pass
+        const uint8_t *tables = slots + NSLOT * SLICE_SLOT;
+        // (addresses that the compiler is not to compute again for each term)
+        uint32_t tb = smem_u32(tables), pb = smem_u32(planes) + (uint32_t)byte0;
+        asm volatile("" : "+r"(tb), "+r"(pb));
         if (warp_any) {
             for (int t = 0; t < nt; ++t) {
-                const SliceTerm &T = terms[t];
-                const uint32_t fl = T.flags, xs = T.xs, tw = T.tab;
+                uint4 T;
+                asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(T.x), "=r"(T.y), "=r"(T.z), "=r"(T.w)
+                             : "r"(tb + (uint32_t)sizeof(SliceValue) * (uint32_t)t));
+                const uint32_t fl = T.y >> 16, xs = T.y & 0xFFFFu, tw = T.x;
+                const uint32_t pl0 = pb + (T.z >> 16) * (uint32_t)plane_bytes;
+                const bool big = __any_sync(~0u, (fl & ST_BIG) != 0), wide = __any_sync(~0u, (fl & ST_WIDE) != 0);
+                const uint32_t base = big ? 0u : tb + tw;
+                constexpr int N = S == 1 ? 1 : 4;
 #pragma unroll
                 for (int h = 0; h < (S == 8 ? 2 : 1); ++h) {
-                    constexpr int N = S == 1 ? 1 : 4;
-                    const uint8_t *pl = planes + (int)T.plane * plane_bytes + byte0 + 16 * h;
+                    const uint32_t pl = pl0 + 16 * h;
                     const uint32_t xw = slice_plane<N>(pl), kw = slice_plane<N>(pl + plane_bytes);
                     const uint32_t xm = xw & 0x7F7F7F7Fu, km = kw & 0x7F7F7F7Fu;
-                    const uint32_t base = fl & ST_BIG ? 0u : tw;
                     uint32_t at[N];
 #pragma unroll
                     for (int k = 0; k < N; ++k) at[k] = __dp4a(km, 8u << (8 * k), byte_of(xm, k) * xs + base);
-                    if (fl & ST_WIDE) {
+                    if (wide) {
                         const uint32_t cw = slice_plane<N>(pl + 2 * plane_bytes);
-                        const uint8_t *lut = chunk + 16 * (int)T.lut_off16;
+                        const uint8_t *lut = tables + 16 * (int)(T.z & 0xFFFFu);
                         const uint32_t cs = (fl & ST_EVEN) ? 16u : 32u;
 #pragma unroll
                         for (int k = 0; k < N; ++k) at[k] += (uint32_t)lut[byte_of(cw, k)] * cs;
                     }
                     // K's bit 1 has swapped the halves of the entry
-                    double a[N], b[N];
-                    if (fl & ST_BIG) {
+                    uint2 a[N], b[N];
+                    if (big) {
 #pragma unroll
                         for (int k = 0; k < N; ++k) {
                             const uint8_t *p = j.image + 16 * (size_t)tw + at[k];
                             const uint8_t *q = (const uint8_t *)((uintptr_t)p ^ 8u);
-                            a[k] = CG ? __ldcg((const double *)p) : __ldg((const double *)p);
-                            b[k] = CG ? __ldcg((const double *)q) : __ldg((const double *)q);
+                            a[k] = CG ? __ldcg((const uint2 *)p) : __ldg((const uint2 *)p);
+                            b[k] = CG ? __ldcg((const uint2 *)q) : __ldg((const uint2 *)q);
                         }
                     } else {
 #pragma unroll
                         for (int k = 0; k < N; ++k) {
-                            a[k] = *(const double *)(chunk + at[k]);
-                            b[k] = *(const double *)(chunk + (at[k] ^ 8u));
+                            a[k] = lds64(at[k]);
+                            b[k] = lds64(at[k] ^ 8u);
                         }
                     }
                     // times i^(K1 + 2 (K2 ^ S)): the signs go to bit 63
                     const uint32_t sI = xw ^ kw, sR = sI ^ (kw << 7);
 #pragma unroll
                     for (int k = 0; k < N; ++k) {
-                        const int ra = (int)((sR << (24 - 8 * k)) & 0x80000000u);
-                        const int ib = (int)((sI << (24 - 8 * k)) & 0x80000000u);
+                        const uint32_t ra = (sR << (24 - 8 * k)) & 0x80000000u, ib = (sI << (24 - 8 * k)) & 0x80000000u;
                         double &re = sre[4 * h + k], &im = sim[4 * h + k];
-                        re = dadd(re, __hiloint2double(__double2hiint(a[k]) ^ ra, __double2loint(a[k])));
-                        im = dadd(im, __hiloint2double(__double2hiint(b[k]) ^ ib, __double2loint(b[k])));
+                        re = dadd(re, __hiloint2double((int)(a[k].y ^ ra), (int)a[k].x));
+                        im = dadd(im, __hiloint2double((int)(b[k].y ^ ib), (int)b[k].x));
                     }
                 }
             }
@@ -686,10 +733,13 @@ __device__ __forceinline__ bool slice_tile(const SampleJob &j, const int64_t s0,
                 put_row(F + k - 1, bit);
             }
         }
-        const int64_t ahead_off = 16 * (int64_t)d.ahead_off16;
-        const uint32_t ahead_bytes = d.ahead_bytes;
+        const int64_t ahead_off = 16 * (int64_t)d.ahead_off16, tab_off = 16 * (int64_t)d.tab_off16;
+        const uint32_t ahead_bytes = d.ahead_bytes, tab_bytes = d.tab_bytes;
         __syncthreads();
-        if (tid == 0 && c + NSLOT < nch) slice_issue(j, ahead_off, ahead_bytes, gc + NSLOT, bar, slots);
+        if (tid == 0 && c + 1 < nch) {
+            slice_issue_tables(j, tab_off, tab_bytes, bar, slots);
+            if (c + NSLOT < nch) slice_issue(j, ahead_off, ahead_bytes, gc + NSLOT, bar, slots);
+        }
     }
     g += (uint32_t)nch;
     if (EVAL >= 0) return true;

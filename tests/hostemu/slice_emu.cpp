@@ -74,7 +74,10 @@ int slice_emu_eval(const ksim_graph_desc *g, int n, int F, int gi, const uint8_t
             const uint8_t *base = s.bytes.data() + c.off;
             for (int t = 0; t < c.n_terms; ++t) {
                 SliceTerm d;
+                SliceValue w;
                 std::memcpy(&d, base + SLICE_HEAD + t * sizeof(SliceTerm), sizeof(d));
+                const uint8_t *tabs = base + c.bytes;
+                std::memcpy(&w, tabs + t * sizeof(SliceValue), sizeof(w));
                 const uint8_t *list = base + 16 * d.list_off16;
                 int r[8], kill = 0, K = 0, y = 0, z = 0, X = 0, S = 0;
                 for (int q = 0; q < d.n_k + d.n_x1 + d.n_x0 + d.n_xp; ++q) {
@@ -102,10 +105,10 @@ int slice_emu_eval(const ksim_graph_desc *g, int n, int F, int gi, const uint8_t
                     }
                 K = (K + 4 * S) & 7;
                 const int e = y + z;
-                const int cls = (d.flags & ST_WIDE) ? base[16 * d.lut_off16 + (y | z << 4)] : e * (e + 1) / 2 + z;
+                const int cls = (d.flags & ST_WIDE) ? tabs[16 * w.lut_off16 + (y | z << 4)] : e * (e + 1) / 2 + z;
                 const int col = (d.flags & ST_EVEN) ? cls : 2 * cls + (K & 1);
-                const size_t at = (size_t)(kill ? 0 : X + 1) * d.xs + (size_t)col * 16;
-                const uint8_t *tab = (d.flags & ST_BIG) ? s.bytes.data() + 16 * (size_t)d.tab : base + d.tab;
+                const size_t at = (size_t)(kill ? 0 : X + 1) * w.xs + (size_t)col * 16;
+                const uint8_t *tab = (d.flags & ST_BIG) ? s.bytes.data() + 16 * (size_t)w.tab : tabs + w.tab;
                 double re, im;
                 std::memcpy(&re, tab + at, 8);
                 std::memcpy(&im, tab + at + 8, 8);

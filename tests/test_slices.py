@@ -119,5 +119,5 @@ def test_not_sliced(emu):
     assert info(emu, [synth.random_graph(rng, 1, 254, 4, 1, 1, 1)], 254)["ok"]
     assert not info(emu, [synth.random_graph(rng, 1, 255, 4, 1, 1, 1)], 255)["ok"]
     empty = synth.random_graph(rng, 0, 10, 4, 1, 1, 1)
-    assert info(emu, [empty], 10) == {"ok": 1, "rows": 10, "planes": 0, "chunks": 1, "bytes": 16, "terms": 0,
+    assert info(emu, [empty], 10) == {"ok": 1, "rows": 10, "planes": 0, "chunks": 1, "bytes": 48, "terms": 0,
                                       "wide": 0, "big": 0}
