@@ -148,14 +148,18 @@ cudaError_t launch_slice_as(const SampleJob &j, int shots, int threads, int tile
 // The tile shape by how many SMs the shots can fill.  Measured on the 40-output
 // t = 12 program (ms; 512 threads x 1 shot at widths 128 / 256 / 512, 512 x 2
 // at 1,024 -- 256 threads x 4, two CTAs an SM -- 256 x 8 at 2,048, two CTAs):
-//    10,000 shots  0.236 0.249 0.267 0.36 0.41 0.68    (19,000 = 148 x 128)
-//    20,000        0.42  0.247 0.269 0.36 0.41 0.68
-//    70,000        0.85  0.49  0.271 0.36 0.41 0.68
-//   100,000        1.26  0.66  0.53  0.363 0.415 0.68
-//   200,000              1.1   0.79  0.72 0.547 0.68   (303,104 = 296 x 1,024)
-//   500,000                    1.84  1.43 1.08 0.92
+//    10,000 shots  0.195 0.202 0.220                     (18,944 = 148 x 128)
+//    37,800        0.387 0.204 0.222 0.275
+//    70,000        0.76  0.40  0.226 0.275 0.300
+//   100,000        1.14  0.60  0.439 0.275 0.300
+//   150,000              0.80  0.446 0.276 0.301 0.506
+//   200,000                          0.541 0.405
+//   303,104                          0.545 0.405 0.506   (= 296 x 1,024)
+//   500,000                                0.793 0.695
 // and alike on the 16-output t = 20 one: the widest tile costs least per shot,
-// but a narrower one that still fits one wave ends sooner.
+// but a narrower one that still fits one wave ends sooner.  Two CTAs of 2,048
+// shots need at most 129 parameter rows; with more (60 outputs, F = 100) one
+// CTA took 1.318 ms for 606,208 shots, two of 1,024 take 1.002.
 template <int EVAL = -1>
 cudaError_t launch_slice(const SampleJob &j, const LaunchCfg &cfg, cudaStream_t st)
 {
@@ -172,7 +176,7 @@ cudaError_t launch_slice(const SampleJob &j, const LaunchCfg &cfg, cudaStream_t 
         return launch_slice_as<1, 512, 1, EVAL>(j, shots, 512, shots, st);
     }
     if (n <= sms * 1024) return launch_slice_as<4, 512, 1, EVAL>(j, 1024, 512, 1024, st);
-    const bool wide = n > 2 * sms * 1024;
+    const bool wide = n > 2 * sms * 1024 && slice_two_ctas(j.s_rows, j.s_planes, 2048);
     const int shots = wide ? 2048 : 1024;
     // equal tiles: a last wave that is nearly empty costs as much as a full one
     const int64_t all = cfg.call_shots > 0 ? cfg.call_shots : j.B;

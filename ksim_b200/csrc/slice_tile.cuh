@@ -37,7 +37,7 @@ namespace ksim {
 // The ring: NSLOT slots of rows, one of tables, a barrier each.
 constexpr int SLICE_RING = NSLOT * SLICE_SLOT + SLICE_TABLES;
 
-// Shared memory of a sliced tile of `shots` (64 to 2,048, a power of two):
+// Shared memory of a sliced tile of `shots` (a power of two up to 2,048):
 // parameter rows, result planes, then the barriers and the ring.
 // (The rows of a 2,048-shot tile are two regions, 1,024 shots each.)
 __host__ __device__ constexpr int slice_region(int rows) { return (rows + 1) * SLICE_ROW; }
@@ -52,6 +52,12 @@ __host__ __device__ constexpr int slice_ring_off(int rows, int planes, int shots
 __host__ __device__ constexpr int slice_smem_bytes(int rows, int planes, int shots)
 {
     return slice_ring_off(rows, planes, shots) + BAR_BYTES + SLICE_RING;
+}
+
+// Two CTAs of a shape fit an SM (228 KB, 1 KB of a CTA reserved).
+__host__ __device__ constexpr bool slice_two_ctas(int rows, int planes, int shots)
+{
+    return 2 * (slice_smem_bytes(rows, planes, shots) + 1024) <= 228 * 1024;
 }
 
 // The most a sliced CTA takes (254 parameters, 2,048 shots): every sliced
@@ -450,7 +456,8 @@ __device__ __forceinline__ uint2 lds64(uint32_t a)
 }
 
 // Sample shots [s0, s_end) of job j in a tile of `shots`, S of them a thread
-// (shots / S threads; the others only share the rows pass).  smem: the CTA's shared
+// (shots / S threads, whole warps: a lane without a shot of the tile would look
+// up result bytes that nothing wrote; the others only share the rows pass).  smem: the CTA's shared
 // memory, parameter rows first, planes at planes_off.  Returns false after a
 // wait timeout (the CTA must then stop using the ring).
 // EVAL: instead of sampling, the job's chunks are one graph's and its rows are
@@ -466,7 +473,7 @@ __device__ __forceinline__ bool slice_tile(const SampleJob &j, const int64_t s0,
     const int plane_bytes = shots;
     const int F = j.F, R = j.s_rows;
     const int region = slice_region(R);
-    constexpr bool ONE = S == 8;
+    constexpr bool ONE = S == 8;  // (S = 8 comes with 2,048 shots)
     const int warp = __shfl_sync(~0u, tid >> 5, 0);  // (the same in all lanes, also to the compiler)
     SliceLane ln;
     ln.L = ONE ? 32 : shots >> 6;

@@ -19,10 +19,10 @@ def _graphs(seed, F, n_out, G=3, **kw):
     return rng, [synth.random_graph(rng, G, F + k, **size) for k in range(n_out + 1)]
 
 
-@pytest.mark.parametrize("F", [5, 16])
+@pytest.mark.parametrize("F", [5, 16, 140])
 def test_tile_shapes(cuda_device, oracle_port, F):
-    """Shot counts around each line of the launch rule, and every tile width a
-    caller can ask for."""
+    """Shot counts around each line of the launch rule (140 parameters: one that
+    keeps the narrower tile), and every tile width a caller can ask for."""
     import torch
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     rng, graphs = _graphs(F, F, 3)
