@@ -23,7 +23,8 @@
 // 32-bit ones, each group by its costliest item — as programmatic dependent
 // launches: each kernel starts once every CTA of the one before it runs, and
 // fills the slots that one frees as it drains, so the classes overlap without
-// the run-to-run dispatch order of concurrent graph branches.  The counter
+// the run-to-run dispatch order of concurrent graph branches.  Classes whose
+// jobs all have sliced streams run one body and draw from one list.  The counter
 // reset and the launches are captured once into a CUDA graph and replayed.
 #include <cuda_runtime.h>
 
@@ -239,6 +240,7 @@ struct BatchClass {
     size_t smem = 0;
     BatchItem *d_items = nullptr;
     int n_items = 0, grid = 0;
+    int n_own = 0;          // of its own jobs (the sliced classes share theirs)
     bool sliced = true;     // every job has a sliced stream
     bool high = false;      // hybrid, general and wide classes: launched before the 32-bit ones
     double head_cost = 0;   // cost of its costliest item
@@ -384,15 +386,18 @@ ksim_status ksim_batch_create(const ksim_batch_job *jobs, int32_t n_jobs, const 
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     // a sliced tile is as wide as the batch allows: 1,024 shots cost least a
-    // shot (one of 512 costs about 0.7 of it, of 256 about 0.55), but an item
-    // longer than a few percent of the whole batch's time would be its tail
+    // shot (one of 512 takes 0.83 as long, of 256 0.75), but an item longer
+    // than the rest of the batch takes would be its tail.  64 programs: 1,024
+    // up to a quarter of the batch's time and 512 up to half of it took 1.86 ms
+    // (the narrow tiles' work, twice what the shots need), up to 0.6 and 1.2 of
+    // it 1.22, once and twice 1.06, 1.5 and 3 times 1.17
     double batch_time = 0;  // in terms of a 1,024-shot tile, per CTA slot
     for (int i = 0; i < n_jobs; ++i)
         batch_time += (double)jobs[i].comp->img.n_terms * ((double)((jobs[i].B + 1023) / 1024)) / (2.0 * std::max(sms, 1));
     auto slice_shots = [&](const ksim_component *c) {
         const double t = (double)c->img.n_terms;
         const int most = b->threads <= 64 ? 512 : 1024;
-        return std::min(most, t <= 0.25 * batch_time ? 1024 : t <= 0.5 * batch_time ? 512 : 256);
+        return std::min(most, t <= batch_time ? 1024 : t <= 2 * batch_time ? 512 : 256);
     };
     std::vector<BatchItem> items[BATCH_CLASSES];
     std::vector<double> cost[BATCH_CLASSES];
@@ -436,7 +441,7 @@ ksim_status ksim_batch_create(const ksim_batch_job *jobs, int32_t n_jobs, const 
             it.shots = (int32_t)tile;
             it.s0 = s0;
             items[cl].push_back(it);
-            cost[cl].push_back(k.sliced ? (double)c->img.n_terms * (tile >= 1024 ? 1.0 : tile >= 512 ? 0.7 : 0.55)
+            cost[cl].push_back(k.sliced ? (double)c->img.n_terms * (tile >= 1024 ? 1.0 : tile >= 512 ? 0.83 : 0.75)
                                         : bytes * (double)std::min<int64_t>(tile, jb.B - s0));
         }
     }
@@ -448,6 +453,26 @@ ksim_status ksim_batch_create(const ksim_batch_job *jobs, int32_t n_jobs, const 
     if (e != cudaSuccess) {
         ksim_batch_destroy(b.release());
         return cuda_fail(e, "batch upload");
+    }
+    // The sliced classes run the same body, so their CTAs share one list and
+    // counter: the longest item of any of them goes first, whichever kernel
+    // its class launches.
+    for (int c = 0; c < BATCH_CLASSES; ++c) b->cls[c].n_own = (int)items[c].size();
+    std::vector<BatchItem> pool;
+    std::vector<double> pool_cost;
+    int pool_counter = 0, pool_ring = 0;
+    for (int c = 0; c < BATCH_CLASSES; ++c) {
+        if (!b->cls[c].sliced || items[c].empty()) continue;
+        pool.insert(pool.end(), items[c].begin(), items[c].end());
+        pool_cost.insert(pool_cost.end(), cost[c].begin(), cost[c].end());
+        pool_counter = c;
+        pool_ring = std::max(pool_ring, b->cls[c].ring_off);
+    }
+    for (int c = 0; c < BATCH_CLASSES; ++c) {
+        if (!b->cls[c].sliced || items[c].empty()) continue;
+        items[c] = pool;
+        cost[c] = pool_cost;
+        b->cls[c].ring_off = pool_ring;
     }
     const bool by_value = b->host_jobs.size() <= (size_t)BATCH_PARAM_JOBS;
     for (int c = 0; c < BATCH_CLASSES; ++c) {
@@ -471,13 +496,13 @@ ksim_status ksim_batch_create(const ksim_batch_job *jobs, int32_t n_jobs, const 
             k.p.reset(new BatchParams());
             std::memset(k.p.get(), 0, sizeof(BatchParams));
             k.p->items = k.d_items;
-            k.p->counter = b->d_counter + c;
+            k.p->counter = b->d_counter + (k.sliced ? pool_counter : c);
             k.p->n_items = k.n_items;
             k.p->slot_bytes = k.sliced ? k.ring_off : k.slot;
             std::copy(b->host_jobs.begin(), b->host_jobs.end(), k.p->jobs);
         } else {
             k.pg.items = k.d_items;
-            k.pg.counter = b->d_counter + c;
+            k.pg.counter = b->d_counter + (k.sliced ? pool_counter : c);
             k.pg.n_items = k.n_items;
             k.pg.slot_bytes = k.sliced ? k.ring_off : k.slot;
             k.pg.gjobs = b->d_jobs;
@@ -551,7 +576,7 @@ ksim_status ksim_batch_info(const ksim_batch *b, int64_t *n_items, int32_t *grid
     int32_t gsum = 0, l = 0;
     for (const BatchClass &k : b->cls)
         if (k.n_items) {
-            n += k.n_items;
+            n += k.n_own;
             gsum += k.grid;
             ++l;
         }
