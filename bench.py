@@ -62,22 +62,22 @@ sys.path.insert(0, str(ROOT))
 METRIC = ("shots/sec at 1 B200, batched+served vs plain, bit-exact Z[ω]; p50/p99 latency")
 L2_FLUSH_BYTES = 256 << 20
 # DRAM bytes per shot of the plain kernel, from one ncu capture of
-# k_sample on the same workload at 262,144 shots (dram__bytes_read.sum +
-# dram__bytes_write.sum), plus the output row the capture's L2 absorbed;
+# k_slice on the same workload at 1,000,000 shots (dram__bytes_read.sum),
+# plus the output row, most of which the capture's L2 absorbed;
 # scaled to a launch by its shots (the capture's command and figures are kept
 # with the ncu summaries under profiles/).
-NCU_DRAM_BYTES_PER_SHOT = {"cfg2-medium-40q-t12": 67.4 + 40.0, "cfg4-large-rank-85q-t20": 61.1 + 16.0}
+NCU_DRAM_BYTES_PER_SHOT = {"cfg2-medium-40q-t12": 65.2 + 40.0, "cfg4-large-rank-85q-t20": 58.6 + 16.0}
 # Thread instructions per shot of the plain kernel on the same workload, from
 # one ncu capture (smsp__thread_inst_executed.sum / shots of the captured
 # launch); the issue roofline of the bench line is this times shots/s over
 # the SMs' issue ceiling (capture command and figures: the ncu summaries
 # under profiles/).
-NCU_THREAD_INST_PER_SHOT = {"cfg2-medium-40q-t12": 138386, "cfg4-large-rank-85q-t20": 201817}
+NCU_THREAD_INST_PER_SHOT = {"cfg2-medium-40q-t12": 27464, "cfg4-large-rank-85q-t20": 32099}
 # Thread instructions of one cfg3 batch (its five class kernels, one ncu
 # capture at the default launch shape: 128 threads, 14 KiB slots); the
 # batched leg's issue fraction is this over its timed batch and the issue
 # ceiling (capture command and figures: the ncu summaries under profiles/).
-NCU_THREAD_INST_PER_BATCH = 88.83e9
+NCU_THREAD_INST_PER_BATCH = 17.88e9
 NCU_BATCH_SHAPE = {"threads": 128, "slot_bytes": 14336, "ctas_per_sm": 0}
 # Gate locations of the workloads' circuits (qubits x depth): one
 # single-qubit Pauli channel each in the noisy end-to-end leg.
@@ -779,8 +779,8 @@ def main():
             "frac": issue / issue_peak if issue else None,
             "issue_frac": issue / issue_peak if issue else None,
             "inst_per_shot": inst,
-            "inst_source": "ncu smsp__thread_inst_executed.sum of k_sample on this workload / shots "
-                           "(one capture of 262,144 shots; summary under profiles/)",
+            "inst_source": "ncu smsp__thread_inst_executed.sum of k_slice on this workload / shots "
+                           "(one capture of 1,000,000 shots; summary under profiles/)",
             "peak_source": f"{sms} SMs x 4 issue slots x 32 lanes x median sampled SM clock "
                            f"({sm_mhz:.0f} MHz)",
             "ops_per_shot": work["ops"],
