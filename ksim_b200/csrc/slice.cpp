@@ -457,6 +457,8 @@ bool build_term(const ksim_graph_desc &g, int t, int zero_row, TermOutBytes &o)
     if (g.pf_has_approx) {
         ar = g.pf_approx_f32[2 * (size_t)t];
         ai = g.pf_approx_f32[2 * (size_t)t + 1];
+        // a dead term's 0 times an infinity or NaN is NaN, but its table row is zero
+        if (!std::isfinite(ar) || !std::isfinite(ai)) return false;
     }
     for (size_t ci = 0; ci < cls.size(); ++ci) {
         const int y = cls[ci].first, z = cls[ci].second;

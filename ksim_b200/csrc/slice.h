@@ -28,8 +28,8 @@
 // two, which commutes with every rounding while the scale stays a normal
 // double, so the doubles are the reference's whatever its halving schedule.
 // A component whose terms are all proven (the reference's int64 cannot wrap,
-// scales normal) and fit the limits below gets a sliced stream; the others
-// keep the term records (zring.cuh).
+// scales normal), have finite approximation factors and fit the limits below
+// gets a sliced stream; the others keep the term records (zring.cuh).
 #pragma once
 #include <stddef.h>
 #include <stdint.h>

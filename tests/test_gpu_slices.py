@@ -81,3 +81,22 @@ def test_term_kinds(cuda_device, oracle_port, G):
         pv = rng.integers(0, 2, size=(333, 10 + k)).astype(np.uint8)
         assert same_bits(kc.eval(k, pv), po.eval(k, pv))
         assert same_bits(kc.eval_abs(k, pv), po.eval_abs(k, pv))
+
+
+def test_non_finite_approximation_factor(cuda_device, oracle_port):
+    """An infinite factor makes a dead term NaN: amplitudes, bits and the
+    status word say so."""
+    from ksim_b200._abi import FLAG_NAN
+    rng, graphs = _graphs(31, 12, 3)
+    for g in graphs:
+        g.np_phases[:, 0] = 0
+        g.pf_has_approx, g.pf_approx = True, np.full(3, 0.5 + 1j, np.complex64)
+    graphs[2].pf_approx[1] = np.inf
+    kc, po = _component(graphs, 12), oracle_port.PortOracle(graphs, 12)
+    f = rng.integers(0, 2, size=(3000, 12)).astype(np.uint8)
+    want, want_amp = po.sample(f, 8, 0, return_amp=True)
+    bits, amp = device_sample(kc, f, 8, 0)
+    assert np.isnan(want_amp).any() and np.array_equal(np.isnan(amp), np.isnan(want_amp))
+    assert np.array_equal(bits, want) and kc.status(reset=True) & FLAG_NAN
+    pv = rng.integers(0, 2, size=(333, 14)).astype(np.uint8)
+    assert np.array_equal(np.isnan(kc.eval_abs(2, pv)), np.isnan(po.eval_abs(2, pv)))

@@ -121,3 +121,20 @@ def test_not_sliced(emu):
     empty = synth.random_graph(rng, 0, 10, 4, 1, 1, 1)
     assert info(emu, [empty], 10) == {"ok": 1, "rows": 10, "planes": 0, "chunks": 1, "bytes": 48, "terms": 0,
                                       "wide": 0, "big": 0}
+
+
+@pytest.mark.parametrize("factor", [complex(np.inf, 0.0), complex(0.0, -np.inf), complex(np.nan, 1.0)])
+def test_non_finite_approximation_factor(emu, factor):
+    """A dead term (value 0) times a factor that is not finite is NaN
+    (zx_eval.hpp:177-178), which the zero row of a value table is not: the
+    component keeps the term records."""
+    rng = np.random.default_rng(9)
+    g = synth.random_graph(rng, 3, 10, 4, 2, 2, 2)
+    g.np_phases[:, 0] = 0  # a row that kills the term
+    g.pf_has_approx = True
+    g.pf_approx = np.full(3, 1.5 - 0.25j, np.complex64)
+    assert info(emu, [g], 10)["ok"]
+    g.pf_approx[1] = factor
+    assert not info(emu, [g], 10)["ok"]
+    g.pf_has_approx = False  # the factors are not read
+    assert info(emu, [g], 10)["ok"]
