@@ -440,7 +440,10 @@ bool build_term(const ksim_graph_desc &g, int t, int zero_row, TermOutBytes &o)
     o.tab.assign(xs * (size_t)(nx + 2), 0);
 
     base.e += R.n_two;
-    for (int i = 0; i < R.n_22; ++i) base = mul(base, k22);
+    for (int i = 0; i < R.n_22; ++i) {
+        base = mul(base, k22);
+        if (!reduce(base)) return false;
+    }
     for (int i = 0; i < R.n_8; ++i) {
         base = mul(base, kKappa);
         if (!reduce(base)) return false;

@@ -138,3 +138,16 @@ def test_non_finite_approximation_factor(emu, factor):
     assert not info(emu, [g], 10)["ok"]
     g.pf_has_approx = False  # the factors are not read
     assert info(emu, [g], 10)["ok"]
+
+
+@pytest.mark.parametrize("n", [24, 60, 86, 112])
+def test_many_products_of_two_plus_two_i(emu, oracle_port, n):
+    """PhasePairs columns with both phases 2 and equal signs contribute
+    (2 + 2i)^n: 2^(1.5 n) before its powers of two are taken out, past 127
+    bits from n = 85."""
+    rng = np.random.default_rng(n)
+    g = synth.random_graph(rng, 2, 10, 4, 1, 1, n, density=0.3)
+    g.ph_alpha[:], g.ph_beta[:], g.ph_counts[:], g.np_phases[:] = 2, 2, n, 1
+    g.ph_alpha_p[:], g.ph_beta_p[:] = 0, 0
+    assert info(emu, [g], 10)["ok"]
+    check(emu, oracle_port, [g], 10, rng)
