@@ -188,8 +188,9 @@ ksim_status ksim_component_set_launch(ksim_component *c, int32_t threads, int32_
                                       int32_t slot_bytes);
 ksim_status ksim_component_get_launch(const ksim_component *c, int32_t *threads, int32_t *staged,
                                       int32_t *slot_bytes);
-/* Bound of the staging waits of this component's sampling kernels (plain,
- * batched, served and allocation-free), in non-blocking polls of the
+/* Bound of the staging waits of this component's kernels (plain, batched,
+ * served and allocation-free sampling; eval and eval_abs of a component with
+ * a sliced stream), in non-blocking polls of the
  * mbarrier 64 ns apart: a wait that runs out raises KSIM_FLAG_WAIT_TIMEOUT,
  * the CTA waits (with the built-in bound) for the copies it issued and leaves
  * without writing its shots, and the synchronous host calls report

@@ -450,13 +450,18 @@ static ksim_status eval_common(ksim_component *c, int32_t graph, const uint8_t *
         s.amp = (double *)c->ws_aux.p;
         s.B = B;
         s.status = c->d_status;
+        s.wait_limit = c->wait_limit;
         e = launch_eval_sliced(s, mode, cfg, c->stream);
         if (e != cudaSuccess) return cuda_fail(e, "eval kernel launch");
         e = cudaMemcpyAsync(out, c->ws_aux.p, out_bytes, cudaMemcpyDeviceToHost, c->stream);
         if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync(eval out)");
-        e = cudaStreamSynchronize(c->stream);
+        // this kernel stages chunks: a wait that ran out left rows unwritten
+        uint32_t flags = 0;
+        e = cudaMemcpyAsync(&flags, c->d_status, sizeof(flags), cudaMemcpyDeviceToHost, c->stream);
+        const cudaError_t end = cudaStreamSynchronize(c->stream);  // (also before leaving `flags` and `out`)
+        if (e == cudaSuccess) e = end;
         if (e != cudaSuccess) return cuda_fail(e, "eval");
-        return KSIM_OK;
+        return report_timeout_flags(c, flags);
     }
     EvalJob j = {};
     j.image = c->d_image;

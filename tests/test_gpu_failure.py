@@ -98,3 +98,22 @@ def test_served_wait_timeout_fails_the_request_only(cuda_device, oracle_port):
         assert np.array_equal(good.result(timeout=120), want)
         st = srv.stats()
     assert st["failed"] == 1 and st["completed"] == 1
+
+
+@pytest.mark.parametrize("call", ["eval", "eval_abs"])
+def test_eval_reports_a_wait_timeout(cuda_device, oracle_port, call):
+    """eval and eval_abs of a component with a sliced stream stage chunks: a
+    wait that runs out fails the call (its rows were not written) and leaves
+    the status word clear; the next call is exact."""
+    from helpers import same_bits
+    comp, kc, _ = _component(912)
+    rng = np.random.default_rng(3)
+    pv = rng.integers(0, 2, size=(5000, 63)).astype(np.uint8)
+    want = getattr(oracle_port.PortOracle(comp.graphs, 60), call)(3, pv)
+    kc.set_wait_limit(1)
+    with pytest.raises(TimeoutError, match="staging wait"):
+        getattr(kc, call)(3, pv)
+    assert kc.status() == 0
+    kc.set_wait_limit(0)
+    assert same_bits(getattr(kc, call)(3, pv), want)
+    assert kc.status() == 0
