@@ -23,8 +23,9 @@
 // 32-bit ones, each group by its costliest item — as programmatic dependent
 // launches: each kernel starts once every CTA of the one before it runs, and
 // fills the slots that one frees as it drains, so the classes overlap without
-// the run-to-run dispatch order of concurrent graph branches.  Classes whose
-// jobs all have sliced streams run one body and draw from one list.  The counter
+// the run-to-run dispatch order of concurrent graph branches.  The jobs of a
+// class that have sliced streams are a group of their own; these groups run
+// one body and draw from one list.  The counter
 // reset and the launches are captured once into a CUDA graph and replayed.
 #include <cuda_runtime.h>
 
@@ -55,9 +56,13 @@ struct BatchItem {
 };
 
 // Classes: 3 (W - 1) + p for W <= 4 (p = 0 32-bit, 1 hybrid, 2 general), 12
-// for W > 4.
+// for W > 4.  Groups: the jobs of a class without a sliced stream, then
+// those with one (BATCH_CLASSES further on): one job without does not take
+// the others of its class off the sliced body (300,000 shots of the 40-output
+// program beside 500 shots of a job without: 0.594 ms; as one class 1.474).
 constexpr int BATCH_CLASSES = 13;
 constexpr int BATCH_WIDE = 12;
+constexpr int BATCH_GROUPS = 2 * BATCH_CLASSES;
 inline int batch_class(int W, int paths)
 {
     if (W > 4) return BATCH_WIDE;
@@ -147,7 +152,7 @@ __global__ void KSIM_BATCH_BOUNDS(PATHS) k_batch_c(const __grid_constant__ PT P)
     pdl_wait();
 }
 
-// A class whose jobs all have sliced streams: the sliced body (one for every W
+// A group of jobs with sliced streams: the sliced body (one for every W
 // and term path), 256 threads, four shots a thread; a tile's width is its
 // item's.
 template <typename PT>
@@ -209,11 +214,11 @@ __global__ void __maxnreg__(255) k_batch_wide(const __grid_constant__ PT P)
     pdl_wait();
 }
 
-// The kernel of class `cls` for job-table type PT.
+// The kernel of group `cls` for job-table type PT.
 template <typename PT>
-const void *batch_kernel(int cls, bool sliced)
+const void *batch_kernel(int cls)
 {
-    if (sliced) return (const void *)k_batch_s<PT>;
+    if (cls >= BATCH_CLASSES) return (const void *)k_batch_s<PT>;
 #define KSIM_BK(WW)                                                                  \
     case 3 * (WW - 1): return (const void *)k_batch_c<PT, WW, PATHS_NARROW>;         \
     case 3 * (WW - 1) + 1: return (const void *)k_batch_c<PT, WW, PATHS_NARROW_HYBRID>; \
@@ -233,7 +238,7 @@ using namespace ksim;
 
 namespace {
 
-// One class of a batch: launch shape and items.
+// One group of a batch: launch shape and items.
 struct BatchClass {
     int threads = 128, slot = 14336, max_w = 1;
     int ring_off = 0;       // of a sliced class: its CTAs' rows and planes
@@ -241,7 +246,7 @@ struct BatchClass {
     BatchItem *d_items = nullptr;
     int n_items = 0, grid = 0;
     int n_own = 0;          // of its own jobs (the sliced classes share theirs)
-    bool sliced = true;     // every job has a sliced stream
+    bool sliced = false;    // its jobs have sliced streams
     bool high = false;      // hybrid, general and wide classes: launched before the 32-bit ones
     double head_cost = 0;   // cost of its costliest item
     std::unique_ptr<BatchParams> p;  // the job table by value (<= BATCH_PARAM_JOBS jobs)
@@ -253,7 +258,7 @@ struct BatchClass {
 struct ksim_batch {
     int device = 0;
     int threads = 128, slot_bytes = 14336, ctas_per_sm = 0, use_graph = 1;  // 32-bit classes (tuned)
-    BatchClass cls[BATCH_CLASSES];
+    BatchClass cls[BATCH_GROUPS];
     std::vector<ksim_component *> comps;
     std::vector<BatchJobDev> host_jobs;
     BatchJobDev *d_jobs = nullptr;
@@ -289,20 +294,20 @@ static cudaError_t batch_launch_class(ksim_batch *b, int c, cudaStream_t st, boo
     lc.numAttrs = follow ? 1 : 0;
     if (k.p) {
         void *args[] = {(void *)k.p.get()};
-        return cudaLaunchKernelExC(&lc, batch_kernel<BatchParams>(c, k.sliced), args);
+        return cudaLaunchKernelExC(&lc, batch_kernel<BatchParams>(c), args);
     }
     void *args[] = {(void *)&k.pg};
-    return cudaLaunchKernelExC(&lc, batch_kernel<BatchParamsG>(c, k.sliced), args);
+    return cudaLaunchKernelExC(&lc, batch_kernel<BatchParamsG>(c), args);
 }
 
 static ksim_status batch_enqueue(ksim_batch *b, cudaStream_t st)
 {
-    cudaError_t e = cudaMemsetAsync(b->d_counter, 0, BATCH_CLASSES * sizeof(int), st);
+    cudaError_t e = cudaMemsetAsync(b->d_counter, 0, BATCH_GROUPS * sizeof(int), st);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(work counter)");
     // the hybrid / general / wide classes first, then the 32-bit ones; within
     // each group the class with the costliest first item first
     std::vector<int> active;
-    for (int c = 0; c < BATCH_CLASSES; ++c)
+    for (int c = 0; c < BATCH_GROUPS; ++c)
         if (b->cls[c].n_items) active.push_back(c);
     std::stable_sort(active.begin(), active.end(), [&](int x, int y) {
         const BatchClass &a = b->cls[x], &z = b->cls[y];
@@ -340,13 +345,14 @@ ksim_status ksim_batch_create(const ksim_batch_job *jobs, int32_t n_jobs, const 
     // KSIM_BATCH_HYB_THREADS, general and wide CTAs of KSIM_BATCH_GEN_THREADS;
     // slots at least the tuned size (16 KiB for general and wide) and every
     // job's largest term
-    for (int c = 0; c < BATCH_CLASSES; ++c) {
+    for (int c = 0; c < BATCH_GROUPS; ++c) {
         BatchClass &k = b->cls[c];
-        const int p = c == BATCH_WIDE ? 3 : c % 3;
+        const int cl = c % BATCH_CLASSES, p = cl == BATCH_WIDE ? 3 : cl % 3;
+        k.sliced = c >= BATCH_CLASSES;
         k.threads = p == 0 ? b->threads : p == 1 ? KSIM_BATCH_HYB_THREADS : KSIM_BATCH_GEN_THREADS;
         k.slot = p >= 2 ? std::max(16384, b->slot_bytes) : b->slot_bytes;
         k.high = p != 0;
-        k.max_w = c == BATCH_WIDE ? 5 : c / 3 + 1;
+        k.max_w = cl == BATCH_WIDE ? 5 : cl / 3 + 1;
     }
     int device = -1;
     for (int i = 0; i < n_jobs; ++i) {
@@ -365,7 +371,7 @@ ksim_status ksim_batch_create(const ksim_batch_job *jobs, int32_t n_jobs, const 
         if (!jb.d_out_cols && jb.out_stride < jb.out_col0 + c->img.n_out)
             return fail(KSIM_ERR_INVALID_ARGUMENT, "job " + std::to_string(i) + ": out_stride too small");
         const int cl = batch_class(c->img.W, c->cfg.paths);
-        BatchClass &k = b->cls[cl];
+        BatchClass &k = b->cls[cl + (c->cfg.sliced ? BATCH_CLASSES : 0)];
         const int64_t need = (c->img.max_term_bytes + 15) & ~int64_t(15);
         // a slot the caller chose must hold the 32-bit jobs' terms; the
         // default and the other classes' slots grow to their largest term
@@ -373,11 +379,10 @@ ksim_status ksim_batch_create(const ksim_batch_job *jobs, int32_t n_jobs, const 
             return fail(KSIM_ERR_INVALID_ARGUMENT, "job " + std::to_string(i) + ": a term record (" +
                                                        std::to_string(c->img.max_term_bytes) +
                                                        " bytes) exceeds slot_bytes");
-        k.sliced = k.sliced && c->cfg.sliced;
         if (need > k.slot) k.slot = (int)std::min<int64_t>(need, 1 << 30);
         k.max_w = std::max(k.max_w, c->img.W);
     }
-    for (int c = 0; c < BATCH_CLASSES; ++c)
+    for (int c = 0; c < BATCH_GROUPS; ++c)
         if (!b->cls[c].sliced && batch_smem_bytes(b->cls[c].slot, b->cls[c].max_w, b->cls[c].threads) > 227 * 1024)
             return fail(KSIM_ERR_UNSUPPORTED, "a term record needs a staging slot of " +
                                                   std::to_string(b->cls[c].slot) + " bytes, beyond shared memory");
@@ -399,12 +404,12 @@ ksim_status ksim_batch_create(const ksim_batch_job *jobs, int32_t n_jobs, const 
         const int most = b->threads <= 64 ? 512 : 1024;
         return std::min(most, t <= batch_time ? 1024 : t <= 2 * batch_time ? 512 : 256);
     };
-    std::vector<BatchItem> items[BATCH_CLASSES];
-    std::vector<double> cost[BATCH_CLASSES];
+    std::vector<BatchItem> items[BATCH_GROUPS];
+    std::vector<double> cost[BATCH_GROUPS];
     for (int i = 0; i < n_jobs; ++i) {
         const ksim_batch_job &jb = jobs[i];
         ksim_component *c = jb.comp;
-        const int cl = batch_class(c->img.W, c->cfg.paths);
+        const int cl = batch_class(c->img.W, c->cfg.paths) + (c->cfg.sliced ? BATCH_CLASSES : 0);
         BatchClass &k = b->cls[cl];
         LaunchCfg cfg;
         cfg.threads = k.threads;
@@ -449,7 +454,7 @@ ksim_status ksim_batch_create(const ksim_batch_job *jobs, int32_t n_jobs, const 
     if (e == cudaSuccess)
         e = cudaMemcpy(b->d_jobs, b->host_jobs.data(), sizeof(BatchJobDev) * b->host_jobs.size(),
                        cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_counter, BATCH_CLASSES * sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_counter, BATCH_GROUPS * sizeof(int));
     if (e != cudaSuccess) {
         ksim_batch_destroy(b.release());
         return cuda_fail(e, "batch upload");
@@ -457,25 +462,25 @@ ksim_status ksim_batch_create(const ksim_batch_job *jobs, int32_t n_jobs, const 
     // The sliced classes run the same body, so their CTAs share one list and
     // counter: the longest item of any of them goes first, whichever kernel
     // its class launches.
-    for (int c = 0; c < BATCH_CLASSES; ++c) b->cls[c].n_own = (int)items[c].size();
+    for (int c = 0; c < BATCH_GROUPS; ++c) b->cls[c].n_own = (int)items[c].size();
     std::vector<BatchItem> pool;
     std::vector<double> pool_cost;
     int pool_counter = 0, pool_ring = 0;
-    for (int c = 0; c < BATCH_CLASSES; ++c) {
+    for (int c = 0; c < BATCH_GROUPS; ++c) {
         if (!b->cls[c].sliced || items[c].empty()) continue;
         pool.insert(pool.end(), items[c].begin(), items[c].end());
         pool_cost.insert(pool_cost.end(), cost[c].begin(), cost[c].end());
         pool_counter = c;
         pool_ring = std::max(pool_ring, b->cls[c].ring_off);
     }
-    for (int c = 0; c < BATCH_CLASSES; ++c) {
+    for (int c = 0; c < BATCH_GROUPS; ++c) {
         if (!b->cls[c].sliced || items[c].empty()) continue;
         items[c] = pool;
         cost[c] = pool_cost;
         b->cls[c].ring_off = pool_ring;
     }
     const bool by_value = b->host_jobs.size() <= (size_t)BATCH_PARAM_JOBS;
-    for (int c = 0; c < BATCH_CLASSES; ++c) {
+    for (int c = 0; c < BATCH_GROUPS; ++c) {
         BatchClass &k = b->cls[c];
         if (items[c].empty()) continue;
         if (k.sliced) k.threads = 256;
@@ -509,7 +514,7 @@ ksim_status ksim_batch_create(const ksim_batch_job *jobs, int32_t n_jobs, const 
         }
         int active = 0;
         if (e == cudaSuccess) {
-            const void *fn = by_value ? batch_kernel<BatchParams>(c, k.sliced) : batch_kernel<BatchParamsG>(c, k.sliced);
+            const void *fn = by_value ? batch_kernel<BatchParams>(c) : batch_kernel<BatchParamsG>(c);
             e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      k.sliced ? SLICE_SMEM_MAX : (int)k.smem);
             if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&active, fn, k.threads, k.smem);
@@ -518,7 +523,7 @@ ksim_status ksim_batch_create(const ksim_batch_job *jobs, int32_t n_jobs, const 
             ksim_batch_destroy(b.release());
             return cuda_fail(e, "batch setup");
         }
-        const int per_sm = (c % 3 == 0 && c != BATCH_WIDE && b->ctas_per_sm > 0)
+        const int per_sm = (c % BATCH_CLASSES % 3 == 0 && c % BATCH_CLASSES != BATCH_WIDE && b->ctas_per_sm > 0)
                                ? std::min(b->ctas_per_sm, std::max(active, 1))
                                : std::max(active, 1);
         k.grid = std::max(1, std::min(per_sm * sms, k.n_items));
