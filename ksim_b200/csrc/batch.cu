@@ -243,9 +243,10 @@ struct BatchClass {
     int threads = 128, slot = 14336, max_w = 1;
     int ring_off = 0;       // of a sliced class: its CTAs' rows and planes
     size_t smem = 0;
-    BatchItem *d_items = nullptr;
+    BatchItem *d_items = nullptr;  // (a sliced group's may be another's: owns_items)
+    bool owns_items = false;
     int n_items = 0, grid = 0;
-    int n_own = 0;          // of its own jobs (the sliced classes share theirs)
+    int n_own = 0;          // of its own jobs (the sliced groups share theirs)
     bool sliced = false;    // its jobs have sliced streams
     bool high = false;      // hybrid, general and wide classes: launched before the 32-bit ones
     double head_cost = 0;   // cost of its costliest item
@@ -459,55 +460,64 @@ ksim_status ksim_batch_create(const ksim_batch_job *jobs, int32_t n_jobs, const 
         ksim_batch_destroy(b.release());
         return cuda_fail(e, "batch upload");
     }
-    // The sliced classes run the same body, so their CTAs share one list and
+    // The sliced groups run the same body, so their CTAs share one list and
     // counter: the longest item of any of them goes first, whichever kernel
-    // its class launches.
+    // takes it.  The group launched first (`lead`) has the list's CTAs, all but
+    // one for each other sliced group: their sum is what occupancy or
+    // ctas_per_sm allows.
     for (int c = 0; c < BATCH_GROUPS; ++c) b->cls[c].n_own = (int)items[c].size();
-    std::vector<BatchItem> pool;
-    std::vector<double> pool_cost;
-    int pool_counter = 0, pool_ring = 0;
+    int lead = -1, n_sliced = 0, pool_ring = 0;
     for (int c = 0; c < BATCH_GROUPS; ++c) {
         if (!b->cls[c].sliced || items[c].empty()) continue;
-        pool.insert(pool.end(), items[c].begin(), items[c].end());
-        pool_cost.insert(pool_cost.end(), cost[c].begin(), cost[c].end());
-        pool_counter = c;
+        if (lead < 0 || (b->cls[c].high && !b->cls[lead].high)) lead = c;
+        ++n_sliced;
         pool_ring = std::max(pool_ring, b->cls[c].ring_off);
     }
     for (int c = 0; c < BATCH_GROUPS; ++c) {
-        if (!b->cls[c].sliced || items[c].empty()) continue;
-        items[c] = pool;
-        cost[c] = pool_cost;
-        b->cls[c].ring_off = pool_ring;
+        if (!b->cls[c].sliced || c == lead || items[c].empty()) continue;
+        items[lead].insert(items[lead].end(), items[c].begin(), items[c].end());
+        cost[lead].insert(cost[lead].end(), cost[c].begin(), cost[c].end());
     }
     const bool by_value = b->host_jobs.size() <= (size_t)BATCH_PARAM_JOBS;
-    for (int c = 0; c < BATCH_GROUPS; ++c) {
+    auto setup = [&](int c) -> cudaError_t {
         BatchClass &k = b->cls[c];
-        if (items[c].empty()) continue;
-        if (k.sliced) k.threads = 256;
+        const bool shared = k.sliced && c != lead;
+        if (k.sliced) {
+            k.threads = 256;
+            k.ring_off = pool_ring;
+        }
         k.smem = k.sliced ? (size_t)k.ring_off + BAR_BYTES + SLICE_RING
                           : batch_smem_bytes(k.slot, k.max_w, k.threads);
-        std::vector<int> order(items[c].size());
-        std::iota(order.begin(), order.end(), 0);
-        std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[c][x] > cost[c][y]; });
-        std::vector<BatchItem> sorted;
-        sorted.reserve(order.size());
-        for (int o : order) sorted.push_back(items[c][o]);
-        k.n_items = (int)sorted.size();
-        k.head_cost = cost[c][order[0]];
-        e = cudaMalloc(&k.d_items, sizeof(BatchItem) * sorted.size());
-        if (e == cudaSuccess)
-            e = cudaMemcpy(k.d_items, sorted.data(), sizeof(BatchItem) * sorted.size(), cudaMemcpyHostToDevice);
+        cudaError_t e = cudaSuccess;
+        if (shared) {
+            k.d_items = b->cls[lead].d_items;
+            k.n_items = b->cls[lead].n_items;
+            k.head_cost = b->cls[lead].head_cost;
+        } else {
+            std::vector<int> order(items[c].size());
+            std::iota(order.begin(), order.end(), 0);
+            std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[c][x] > cost[c][y]; });
+            std::vector<BatchItem> sorted;
+            sorted.reserve(order.size());
+            for (int o : order) sorted.push_back(items[c][o]);
+            k.n_items = (int)sorted.size();
+            k.head_cost = cost[c][order[0]];
+            e = cudaMalloc(&k.d_items, sizeof(BatchItem) * sorted.size());
+            k.owns_items = e == cudaSuccess;
+            if (e == cudaSuccess)
+                e = cudaMemcpy(k.d_items, sorted.data(), sizeof(BatchItem) * sorted.size(), cudaMemcpyHostToDevice);
+        }
         if (by_value) {
             k.p.reset(new BatchParams());
             std::memset(k.p.get(), 0, sizeof(BatchParams));
             k.p->items = k.d_items;
-            k.p->counter = b->d_counter + (k.sliced ? pool_counter : c);
+            k.p->counter = b->d_counter + (k.sliced ? lead : c);
             k.p->n_items = k.n_items;
             k.p->slot_bytes = k.sliced ? k.ring_off : k.slot;
             std::copy(b->host_jobs.begin(), b->host_jobs.end(), k.p->jobs);
         } else {
             k.pg.items = k.d_items;
-            k.pg.counter = b->d_counter + (k.sliced ? pool_counter : c);
+            k.pg.counter = b->d_counter + (k.sliced ? lead : c);
             k.pg.n_items = k.n_items;
             k.pg.slot_bytes = k.sliced ? k.ring_off : k.slot;
             k.pg.gjobs = b->d_jobs;
@@ -519,14 +529,21 @@ ksim_status ksim_batch_create(const ksim_batch_job *jobs, int32_t n_jobs, const 
                                      k.sliced ? SLICE_SMEM_MAX : (int)k.smem);
             if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&active, fn, k.threads, k.smem);
         }
-        if (e != cudaSuccess) {
-            ksim_batch_destroy(b.release());
-            return cuda_fail(e, "batch setup");
-        }
-        const int per_sm = (c % BATCH_CLASSES % 3 == 0 && c % BATCH_CLASSES != BATCH_WIDE && b->ctas_per_sm > 0)
+        if (e != cudaSuccess) return e;
+        const int cl = c % BATCH_CLASSES;
+        const int per_sm = ((k.sliced || (cl % 3 == 0 && cl != BATCH_WIDE)) && b->ctas_per_sm > 0)
                                ? std::min(b->ctas_per_sm, std::max(active, 1))
                                : std::max(active, 1);
-        k.grid = std::max(1, std::min(per_sm * sms, k.n_items));
+        const int ctas = per_sm * sms - (c == lead ? n_sliced - 1 : 0);
+        k.grid = shared ? 1 : std::max(1, std::min(ctas, k.n_items));
+        return cudaSuccess;
+    };
+    if (lead >= 0) e = setup(lead);
+    for (int c = 0; c < BATCH_GROUPS && e == cudaSuccess; ++c)
+        if (c != lead && !items[c].empty()) e = setup(c);
+    if (e != cudaSuccess) {
+        ksim_batch_destroy(b.release());
+        return cuda_fail(e, "batch setup");
     }
     *out = b.release();
     return KSIM_OK;
@@ -599,7 +616,7 @@ void ksim_batch_destroy(ksim_batch *b)
     batch_drop_graph(b);
     if (b->cap_stream) cudaStreamDestroy(b->cap_stream);
     for (BatchClass &k : b->cls) {
-        if (k.d_items) cudaFree(k.d_items);
+        if (k.owns_items) cudaFree(k.d_items);
     }
     if (b->d_jobs) cudaFree(b->d_jobs);
     if (b->d_counter) cudaFree(b->d_counter);

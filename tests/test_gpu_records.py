@@ -36,3 +36,20 @@ def test_batch_class_with_and_without_sliced_streams(cuda_device, oracle_port):
     assert records + -(-shots[0] // 1024) <= bs.info()["items"] <= records + -(-shots[0] // 256)
     for i in (0, 1):
         assert _batch(comps[i:i + 1], shots[i:i + 1])[2].info()["launches"] == 1
+
+
+@pytest.mark.parametrize("per_sm", [0, 1])
+def test_batch_ctas_per_sm(cuda_device, oracle_port, per_sm):
+    """ctas_per_sm bounds the persistent CTAs of the sliced jobs together,
+    whichever of their classes they belong to."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    comps = [unsliced.component(k, F, sliced=True) for k, F in (("narrow", 20), ("hybrid", 60), ("all", 60), ("all", 124))]
+    progs, fs, bs = _batch(comps, [200_000] * 4)
+    bs._build({"threads": 128, "slot_bytes": 14336, "ctas_per_sm": per_sm})
+    assert bs.info()["launches"] == 4
+    assert bs.info()["grid"] == (2 - per_sm) * sms
+    for i, got in enumerate(bs.sample(fs)):
+        assert np.array_equal(got[:3000], oracle_port.program_sample(progs[i], fs[i][:3000], i)), i
+        rest = bs.samplers[i].sample(fs[i], i)
+        assert np.array_equal(got, rest), i
