@@ -37,6 +37,7 @@
 #include <vector>
 
 #include "../../include/ksim_b200.h"
+#include "batch_plan.h"
 #include "kernels.h"
 #include "runtime.h"
 #include "sample_tile.cuh"
@@ -249,7 +250,7 @@ struct BatchClass {
     int n_own = 0;          // of its own jobs (the sliced groups share theirs)
     bool sliced = false;    // its jobs have sliced streams
     bool high = false;      // hybrid, general and wide classes: launched before the 32-bit ones
-    double head_cost = 0;   // cost of its costliest item
+    double head_cost = 0;   // cost of its costliest item, in us
     std::unique_ptr<BatchParams> p;  // the job table by value (<= BATCH_PARAM_JOBS jobs)
     BatchParamsG pg = {};            // otherwise through a pointer
 };
@@ -447,8 +448,8 @@ ksim_status ksim_batch_create(const ksim_batch_job *jobs, int32_t n_jobs, const 
             it.shots = (int32_t)tile;
             it.s0 = s0;
             items[cl].push_back(it);
-            cost[cl].push_back(k.sliced ? (double)c->img.n_terms * (tile >= 1024 ? 1.0 : tile >= 512 ? 0.83 : 0.75)
-                                        : bytes * (double)std::min<int64_t>(tile, jb.B - s0));
+            cost[cl].push_back(k.sliced ? slice_item_us(c->img.n_terms, (int)tile)
+                                        : record_item_us(bytes, std::min<int64_t>(tile, jb.B - s0)));
         }
     }
     cudaError_t e = cudaMalloc(&b->d_jobs, sizeof(BatchJobDev) * b->host_jobs.size());
