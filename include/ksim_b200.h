@@ -363,7 +363,8 @@ typedef struct ksim_server_stats {
     int64_t submitted, completed, failed, cancelled;
     int64_t shots_completed;
     int64_t loop_launches;   /* launches of the device-resident loop kernel */
-    int64_t side_launches;   /* programs with > 256 parameter bits run as plain launches */
+    int64_t side_launches;   /* requests run as plain launches: a component without a sliced
+                                stream and with > 256 parameter bits or a term beyond the slots */
     int64_t pending, in_flight;
     int64_t arena_in_use, arena_capacity;
 } ksim_server_stats;

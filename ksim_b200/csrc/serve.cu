@@ -7,8 +7,9 @@
 // the next, so the tiles of every request admitted so far are handed out in
 // arrival order while earlier requests are still running on other CTAs.  The
 // CTA copies the job's descriptor into shared memory with L2-only loads and
-// runs the sliced sampling tile (slice_tile.cuh, L2-coherent loads, one staging
-// ring per CTA for its whole life).  The CTA that finishes a job's last tile
+// runs the sliced sampling tile (slice_tile.cuh), or the term-record tile
+// (sample_tile.cuh) of a component without a sliced stream, with L2-coherent
+// loads and one staging ring of each kind per CTA for its whole life.  The CTA that finishes a job's last tile
 // decrements the request's job count; the one that finishes the request
 // writes the request's sequence number into a host-mapped flag after a
 // system-scope fence.  With nothing to claim, thread 0 backs off with
@@ -30,9 +31,10 @@
 //   3. polls the completion flags, copies finished outputs (and the request's
 //      status word) to the caller's buffer on a second copy stream, and frees
 //      the request's resources once that copy is done.
-// Programs with a component that has no sliced stream (more than 254
-// parameters, terms without a range proof) run as plain launches on a side
-// stream, admitted and completed through the same queue.
+// Programs with a component that has no sliced stream and more than 256
+// parameter bits (W > 4), or a term record beyond the loop's slots, run as plain
+// launches on a side stream, admitted and completed through the same queue.
+// (The loop's CTAs fill the SMs, so such a launch waits for them to go idle.)
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -60,8 +62,9 @@ struct ServeJob {
     int32_t shots, n_tiles;  // shots of a tile
     int32_t next_tile;  // tiles handed out (atomic)
     int32_t remaining;  // tiles not finished (atomic)
-    int32_t req_slot, pad0;
-    int64_t pad1;
+    int32_t req_slot;
+    int32_t W;          // parameter words of a term-record job, 0 of a sliced one
+    int32_t paths, pad0;  // its term paths (LaunchCfg::paths)
 };
 static_assert(sizeof(SampleJob) % 16 == 0, "SampleJob is copied in 16-byte words");
 static_assert(sizeof(ServeJob) % 16 == 0, "ServeJob table entries stay 16-byte aligned");
@@ -103,17 +106,54 @@ __device__ __forceinline__ T vload(const T *p)
 constexpr int SERVE_THREADS = 256;
 constexpr int SERVE_SHOTS = 1024;  // widest tile
 constexpr int SERVE_RING = slice_ring_off(SLICE_MAX_ROWS, SLICE_MAX_PLANES, SERVE_SHOTS);
-constexpr int SERVE_SMEM = slice_smem_bytes(SLICE_MAX_ROWS, SLICE_MAX_PLANES, SERVE_SHOTS);
+// A term-record tile has its parity scratch where the rows and planes are, its
+// slots where the sliced ring's are (both written by copies only), and barriers
+// and a chunk count of its own behind them.
+constexpr int SERVE_RECORD_BARS = slice_smem_bytes(SLICE_MAX_ROWS, SLICE_MAX_PLANES, SERVE_SHOTS);
+constexpr int SERVE_SMEM = SERVE_RECORD_BARS + BAR_BYTES;
+constexpr int SERVE_SLOT_MAX = SLICE_RING / NSLOT;
+static_assert(SERVE_RING % 128 == 0 && SERVE_RECORD_BARS % 128 == 0, "alignment");
+static_assert(sliced_smem_bytes(4, SERVE_THREADS) <= (size_t)SERVE_RING, "parity scratch");
+
+// A tile of a term-record job with the body compiled for its W and term paths,
+// out of line: a call costs such a body about a tenth of its speed, but the
+// sliced body, which carries most requests, stays the loop's own.
+template <int W, int PATHS>
+__device__ __noinline__ bool serve_record_body(const SampleJob &j, int64_t s0, uint64_t *bar, uint8_t *slots,
+                                               uint32_t &g, uint8_t *scratch)
+{
+    return sample_tile<W, true, true, shots_per_thread(W), PATHS>(j, s0, bar, slots, g, scratch);
+}
+template <int W>
+__device__ __forceinline__ bool serve_record_w(int paths, const SampleJob &j, int64_t s0, uint64_t *bar,
+                                               uint8_t *slots, uint32_t &g, uint8_t *scratch)
+{
+    if (paths == PATHS_NARROW) return serve_record_body<W, PATHS_NARROW>(j, s0, bar, slots, g, scratch);
+    if (paths == PATHS_NARROW_HYBRID)
+        return serve_record_body<W, PATHS_NARROW_HYBRID>(j, s0, bar, slots, g, scratch);
+    return serve_record_body<W, PATHS_ALL>(j, s0, bar, slots, g, scratch);
+}
+__device__ __noinline__ bool serve_record_tile(int W, int paths, const SampleJob &j, int64_t s0, uint64_t *bar,
+                                               uint8_t *slots, uint32_t &g, uint8_t *scratch)
+{
+    switch (W) {
+    case 1: return serve_record_w<1>(paths, j, s0, bar, slots, g, scratch);
+    case 2: return serve_record_w<2>(paths, j, s0, bar, slots, g, scratch);
+    case 3: return serve_record_w<3>(paths, j, s0, bar, slots, g, scratch);
+    default: return serve_record_w<4>(paths, j, s0, bar, slots, g, scratch);
+    }
+}
 
 __global__ void __launch_bounds__(SERVE_THREADS, 2) k_serve(ServeJob *jobs, ServeReqDev *reqs, const unsigned long long *ring,
                                                int ring_cap, ServeCtl *ctl, uint32_t *done_flags, long long idle_ns)
 {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ __align__(16) SampleJob s_job;
-    __shared__ int s_slot, s_tile, s_shots;
-    uint64_t *bar = (uint64_t *)(smem + SERVE_RING);
+    __shared__ int s_slot, s_tile, s_shots, s_W, s_paths;
+    uint64_t *bar = (uint64_t *)(smem + SERVE_RING), *record_bar = (uint64_t *)(smem + SERVE_RECORD_BARS);
     slice_ring_init(bar);
-    uint32_t g = 0;
+    ring_init(record_bar);
+    uint32_t g = 0, record_g = 0;
     const long long t_start = global_ns();
     unsigned backoff = 64;
     for (;;) {
@@ -136,6 +176,8 @@ __global__ void __launch_bounds__(SERVE_THREADS, 2) k_serve(ServeJob *jobs, Serv
                 backoff = 64;
                 *(volatile long long *)&ctl->last_claim_ns = global_ns();
                 s_shots = vload(&jobs[slot].shots);
+                s_W = vload(&jobs[slot].W);
+                s_paths = vload(&jobs[slot].paths);
             } else {
                 const long long now = global_ns();
                 const long long last = vload(&ctl->last_claim_ns);
@@ -163,9 +205,11 @@ __global__ void __launch_bounds__(SERVE_THREADS, 2) k_serve(ServeJob *jobs, Serv
         if (slot >= 0) {
             const int shots = s_shots;
             const int64_t s0 = (int64_t)s_tile * shots;
-            const bool ok = slice_tile<4, true>(s_job, s0, s0 + shots < s_job.B ? s0 + shots : s_job.B, shots, smem,
-                                                slice_rows_bytes(s_job.s_rows, shots), bar,
-                                                smem + SERVE_RING + BAR_BYTES, g);
+            uint8_t *slots = smem + SERVE_RING + BAR_BYTES;
+            const bool ok =
+                s_W == 0 ? slice_tile<4, true>(s_job, s0, s0 + shots < s_job.B ? s0 + shots : s_job.B, shots, smem,
+                                               slice_rows_bytes(s_job.s_rows, shots), bar, slots, g)
+                         : serve_record_tile(s_W, s_paths, s_job, s0, record_bar, slots, record_g, smem);
             __threadfence();  // this thread's outputs before the counters below
             __syncthreads();
             if (threadIdx.x == 0) {
@@ -223,7 +267,7 @@ using namespace ksim;
 struct ksim_server {
     int device = 0;
     ksim_server_config cfg = {};
-    LaunchCfg lcfg;
+    LaunchCfg lcfg, record_cfg;  // of sliced jobs, of term-record jobs
     int grid = 0;
 
     uint8_t *d_arena = nullptr;
@@ -326,7 +370,6 @@ ksim_status admit(ksim_server *s, ServeRequest *r)
     // ones, which cost least a shot
     const int64_t by_shots = r->B <= 128 ? 128 : r->B <= 1024 ? 256 : r->B <= 8192 ? 512 : SERVE_SHOTS;
     const int64_t tile = s->cfg.threads > 0 ? std::min<int64_t>(by_shots, 4 * s->cfg.threads) : by_shots;
-    const int64_t tiles = (r->B + tile - 1) / tile;
     std::vector<int> new_jobs;
     for (size_t k = 0; k < p->parts.size(); ++k) {
         ksim_component *c = p->parts[k].comp;
@@ -337,8 +380,12 @@ ksim_status admit(ksim_server *s, ServeRequest *r)
         s->jobs_in_flight += 1;
         ServeJob &J = s->h_jobs[js];
         J = ServeJob();
-        ksim_status st = component_job(c, s->lcfg, J.j);
+        ksim_status st = component_job(c, c->cfg.sliced ? s->lcfg : s->record_cfg, J.j);
         if (st != KSIM_OK) return st;
+        J.W = c->cfg.sliced ? 0 : c->img.W;
+        J.paths = c->cfg.paths;
+        const int64_t shots = c->cfg.sliced ? tile : SERVE_THREADS * shots_per_thread(4);
+        const int64_t tiles = (r->B + shots - 1) / shots;
         J.j.rng_mode = r->rng_mode;
         const ProgramPart &part = p->parts[k];
         J.j.f = part.sel0 > 0 ? d_f + part.sel0 : d_f;
@@ -353,7 +400,7 @@ ksim_status admit(ksim_server *s, ServeRequest *r)
         J.j.shot_offset = 0;
         J.j.seed = r->seed + 0x9E37ull * (uint64_t)k;
         J.j.status = &s->d_reqs[r->slot].flags;
-        J.shots = (int32_t)tile;
+        J.shots = (int32_t)shots;
         J.n_tiles = (int32_t)tiles;
         J.next_tile = 0;
         J.remaining = (int32_t)tiles;
@@ -572,6 +619,9 @@ ksim_status ksim_server_create(const ksim_server_config *cfg_in, ksim_server **o
     // the caller's threads set the widest tile (a power of two)
     s->cfg.threads = threads_given ? (cfg.threads >= 256 ? 256 : cfg.threads >= 128 ? 128 : cfg.threads >= 64 ? 64 : 32) : 0;
     s->lcfg.sliced = 1;
+    s->record_cfg.threads = SERVE_THREADS;
+    s->record_cfg.staged = 1;
+    s->record_cfg.slot_bytes = std::min(cfg.slot_bytes, SERVE_SLOT_MAX);
     s->ring_cap = cfg.max_jobs;
     DeviceGuard g(cfg.device);
     if (!g.ok) return fail(KSIM_ERR_INVALID_ARGUMENT, "cannot select device " + std::to_string(cfg.device));
@@ -653,9 +703,11 @@ ksim_status ksim_server_submit(ksim_server *s, ksim_program *p, const uint8_t *f
     r->out_bytes = B * p->n_outputs;
     r->seed = seed;
     r->rng_mode = rng_mode;
-    // the loop runs sliced streams; a program with a component that has none
-    // runs as plain launches
-    for (const ProgramPart &part : p->parts) r->loop = r->loop && part.comp->cfg.sliced;
+    // the loop runs sliced streams, and term records of up to 4 words that fit
+    // its slots; a program with another component runs as plain launches
+    for (const ProgramPart &part : p->parts)
+        r->loop = r->loop && (part.comp->cfg.sliced ||
+                              (part.comp->img.W <= 4 && part.comp->img.max_term_bytes <= s->record_cfg.slot_bytes));
     for (const ProgramPart &part : p->parts) r->n_jobs += part.comp->img.n_out > 0 ? 1 : 0;
     r->t_submit = Clock::now();
     std::lock_guard<std::mutex> lk(s->mu);

@@ -53,3 +53,25 @@ def test_batch_ctas_per_sm(cuda_device, oracle_port, per_sm):
         assert np.array_equal(got[:3000], oracle_port.program_sample(progs[i], fs[i][:3000], i)), i
         rest = bs.samplers[i].sample(fs[i], i)
         assert np.array_equal(got, rest), i
+
+
+def test_served_term_records_stay_in_the_loop(cuda_device, oracle_port):
+    """Programs of up to 256 parameter bits without a sliced stream run in the
+    device loop beside sliced ones (every W and set of term paths), bit for
+    bit; none is a plain launch, which would wait for the loop to go idle."""
+    from ksim_b200.serve import Server
+    rng = np.random.default_rng(5)
+    reqs = []
+    for k in unsliced.KINDS:
+        for F in (20, 60, 124, 188, 250):  # W = 1, 2 (61 + 3 parameters), 2, 3, 4
+            for sliced in (False, True):
+                prog = synth.single_component_program(unsliced.component(k, F, sliced=sliced))
+                for B in (1, 513, 2000):
+                    reqs.append((prog, synth.sample_f(rng, B, F, 0.1), len(reqs)))
+    with Server(device=0, idle_us=2000) as srv:
+        handles = [srv.submit(p, f, seed) for p, f, seed in reqs]
+        got = [h.result(timeout=120) for h in handles]
+        st = srv.stats()
+    assert st["failed"] == 0 and st["completed"] == len(reqs) and st["side_launches"] == 0
+    for (p, f, seed), g in zip(reqs, got):
+        assert np.array_equal(g, oracle_port.program_sample(p, f, seed))
