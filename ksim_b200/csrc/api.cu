@@ -10,6 +10,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <new>
 #include <numeric>
 #include <string>
 #include <vector>
@@ -207,13 +208,26 @@ ksim_status ksim_component_create(const ksim_graph_desc *graphs, int32_t n_graph
     e = cudaMemcpy(c->d_image, c->img.bytes.data(), c->img.bytes.size(), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpy(program image)");
     SliceImage sl;
-    build_slices(graphs, c->img, sl);
+    try {
+        build_slices(graphs, c->img, sl);
+    } catch (const std::bad_alloc &) {  // (here and below: the term records do without the stream)
+        sl = SliceImage();
+    }
     if (sl.ok) {
         const size_t at = (sl.bytes.size() + 31) & ~size_t(31);
         sl.bytes.resize(at + sl.chunks.size() * sizeof(ChunkDir), 0);
         std::memcpy(sl.bytes.data() + at, sl.chunks.data(), sl.chunks.size() * sizeof(ChunkDir));
         e = cudaMalloc(&c->d_slices, sl.bytes.size());
-        if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(sliced stream)");
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            c->d_slices = nullptr;
+            sl.ok = false;
+        } else if (e != cudaSuccess) {
+            return cuda_fail(e, "cudaMalloc(sliced stream)");
+        }
+    }
+    if (sl.ok) {
+        const size_t at = sl.bytes.size() - sl.chunks.size() * sizeof(ChunkDir);
         e = cudaMemcpy(c->d_slices, sl.bytes.data(), sl.bytes.size(), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpy(sliced stream)");
         c->d_slice_dir = (const ChunkDir *)(c->d_slices + at);

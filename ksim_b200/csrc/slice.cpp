@@ -498,7 +498,7 @@ bool build_term(const ksim_graph_desc &g, int t, int zero_row, TermOutBytes &o)
 
 }  // namespace
 
-void build_slices(const ksim_graph_desc *gs, const HostImage &img, SliceImage &out)
+void build_slices(const ksim_graph_desc *gs, const HostImage &img, SliceImage &out, size_t max_bytes)
 {
     out = SliceImage();
     int rows = img.F + img.n_out;
@@ -585,6 +585,7 @@ void build_slices(const ksim_graph_desc *gs, const HostImage &img, SliceImage &o
             out.bytes.insert(out.bytes.end(), tabs.begin(), tabs.end());
             out.max_planes = std::max(out.max_planes, planes);
             out.chunks.push_back(c);
+            if (out.bytes.size() + big.size() > max_bytes) return;
         } while (t < g.G);
     }
     for (size_t i = 0; i < out.chunks.size(); ++i) {

@@ -50,6 +50,11 @@ constexpr int SLICE_TABLES = 32768;   // bytes of its tables (one slot)
 constexpr int SLICE_MAX_PLANES = 16;  // result bytes per shot of a chunk's terms
 constexpr int SLICE_MAX_TERMS = 8;    // of a chunk
 constexpr int SLICE_AHEAD = 2;        // chunks staged at once
+// A stream's size is bounded: a term's table can take 550 KB (127 lambda steps,
+// 136 classes) where its record takes 4, and building it grows alike (20,000
+// terms of 15 p / q columns: 0.93 GB, 3.9 s, their records 83 MB, 0.9 s).  Up to
+// the bound it pays: 200,000 shots of those take 31 ms, from the records 115.
+constexpr size_t SLICE_MAX_BYTES = (size_t)1 << 30;
 
 // A chunk has two parts, staged by copies of their own: the rows (this head,
 // its terms' SliceTerm, group lists and groups) and, behind them, the tables
@@ -115,7 +120,9 @@ struct SliceImage {
 };
 
 // Build the sliced stream of a component whose image is `img` (build_image on
-// the same descriptors).  out.ok is false when a term does not qualify.
-void build_slices(const ksim_graph_desc *gs, const HostImage &img, SliceImage &out);
+// the same descriptors).  out.ok is false when a term does not qualify or the
+// stream would take more than max_bytes.
+void build_slices(const ksim_graph_desc *gs, const HostImage &img, SliceImage &out,
+                  size_t max_bytes = SLICE_MAX_BYTES);
 
 }  // namespace ksim

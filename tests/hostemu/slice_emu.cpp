@@ -55,6 +55,16 @@ int slice_emu_info(const ksim_graph_desc *g, int n, int F, int64_t *info)
     return 0;
 }
 
+// Size of the stream built under a bound, or 0 if it does not fit.
+int64_t slice_emu_bytes(const ksim_graph_desc *g, int n, int F, int64_t max_bytes)
+{
+    HostImage img;
+    if (build_image(g, n, F, img, g_err)) return -1;
+    SliceImage s;
+    build_slices(g, img, s, (size_t)max_bytes);
+    return s.ok ? (int64_t)s.bytes.size() : 0;
+}
+
 // Complex amplitude of graph gi for B explicit parameter rows.
 int slice_emu_eval(const ksim_graph_desc *g, int n, int F, int gi, const uint8_t *params, int64_t B, int64_t P,
                    double *out)

@@ -151,3 +151,20 @@ def test_many_products_of_two_plus_two_i(emu, oracle_port, n):
     g.ph_alpha_p[:], g.ph_beta_p[:] = 0, 0
     assert info(emu, [g], 10)["ok"]
     check(emu, oracle_port, [g], 10, rng)
+
+
+def test_stream_size_bound(emu):
+    """A stream beyond the bound is not built (its component keeps the term
+    records); tables kept in global memory count too."""
+    rng = np.random.default_rng(11)
+    gs = [synth.random_graph(rng, 6, 10 + k, 45, 2, 2, 15, density=0.4) for k in range(3)]
+    for g in gs:
+        g.ph_alpha[:] = 2 * rng.integers(0, 4, size=g.ph_alpha.shape) + 1
+        g.ph_beta[:] = 2 * rng.integers(0, 4, size=g.ph_beta.shape) + 1
+        g.ph_counts[:] = 15
+    descs, keep = _descs(gs)
+    f = emu.slice_emu_bytes
+    f.restype, f.argtypes = ctypes.c_int64, [*emu.slice_emu_info.argtypes[:3], ctypes.c_int64]
+    full = f(descs, 3, 10, 1 << 30)
+    assert info(emu, gs, 10)["big"] == 18 and full == info(emu, gs, 10)["bytes"] > 18 * 16384
+    assert f(descs, 3, 10, full) == full and f(descs, 3, 10, full - 16384) == 0 and f(descs, 3, 10, 0) == 0
