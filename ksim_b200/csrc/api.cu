@@ -771,18 +771,13 @@ ksim_status program_sample_host(ksim_program *p, const uint8_t *f, int64_t B, in
     uint8_t *d_in = packed ? (uint8_t *)p->ws_fp.p : d_f;       // where the host rows land
     uint8_t *d_back = packed ? (uint8_t *)p->ws_op.p : d_out;   // what goes back
 
-    // sliced kernels that outlast the copies: chunks that fill the SMs; else
-    // (copies dominate, or other kernels) the ramped plan
-    bool sliced = true;
-    double kernel_us = 0;  // of one tile per SM: 0.9 us a term, 1.2 a graph
+    HostCall call = {B, noise ? 0 : f_row, o_row, true, 0, 0, p->sms};
     for (const ProgramPart &part : p->parts) {
-        sliced = sliced && (part.comp->cfg.sliced || part.comp->img.n_out == 0);
-        kernel_us += 0.9 * (double)part.comp->img.n_terms + 1.2 * (double)part.comp->img.n_graphs;
+        call.sliced = call.sliced && (part.comp->d_slices || part.comp->img.n_out == 0);
+        call.n_terms += part.comp->img.n_terms;
+        call.n_graphs += part.comp->img.n_graphs;
     }
-    const double copy_us = (double)B * (double)((noise ? 0 : f_row) + o_row) / 5e4;  // at 50 GB/s
-    const bool fill = sliced && 4 * kernel_us > copy_us;
-    const std::vector<int64_t> bounds = fill ? slice_chunk_bounds(B, p->sms)
-                                             : host_chunk_bounds(B, (noise ? 0 : f_row) + o_row);
+    const std::vector<int64_t> bounds = host_call_bounds(call);
     const int n_chunks = (int)bounds.size() - 1;
     const int lag = host_copy_lag(bounds, p->wave_shots, KSIM_HOST_STREAMS);
     std::vector<cudaEvent_t> &ev_in = p->ev_in, &ev_done = p->ev_done;

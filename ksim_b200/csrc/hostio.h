@@ -52,6 +52,37 @@ inline std::vector<int64_t> slice_chunk_bounds(int64_t B, int64_t sms)
     return b;
 }
 
+// The chunk plan of a call.  sliced: every component with outputs runs the
+// sliced kernel.  n_terms, n_graphs: of all components.
+struct HostCall {
+    int64_t B, in_row, out_row;  // shots; bytes a shot copied in and out
+    bool sliced;
+    int64_t n_terms, n_graphs;
+    int64_t sms;
+};
+
+// Sliced kernels take about kernel_us however few shots a launch has (one tile
+// on each SM), so SM-filling chunks serve them best until copies take several
+// times that: up to 4 kernel_us of them the ramp, which ends on smaller copies,
+// was slower (1 to 60 outputs, 100,000 to 400,000 shots: by 2 to 25 %), beyond it
+// the filling chunks were (1,000,000 shots: by 3 to 11 %).
+// A call of one filling chunk overlaps nothing.  Where its copies outlast the
+// kernel and 2 MiB or more go out, the ramp's smaller chunks hide output copies
+// (60 outputs, 190 f columns, 50,000 shots: 6 % less from pinned buffers, 8 %
+// from pageable ones); with less to hide they cost 2 to 15 % (20 outputs, 64 f
+// columns, 75,000 shots: 7 %).
+inline std::vector<int64_t> host_call_bounds(const HostCall &c)
+{
+    const int64_t row = c.in_row + c.out_row;
+    if (!c.sliced) return host_chunk_bounds(c.B, row);
+    const double kernel_us = 0.9 * (double)c.n_terms + 1.2 * (double)c.n_graphs;
+    const double copy_us = (double)c.B * (double)row / 5e4;  // at 50 GB/s
+    std::vector<int64_t> fill = slice_chunk_bounds(c.B, c.sms);
+    const bool ramp = fill.size() == 2 ? c.B * c.out_row >= ((int64_t)2 << 20) && kernel_us < copy_us
+                                       : 4 * kernel_us <= copy_us;
+    return ramp ? host_chunk_bounds(c.B, row) : fill;
+}
+
 // How many chunks behind the sampling a call issues each chunk's output
 // copy: one wave of sampling CTAs (wave_shots) over the largest chunk,
 // between 1 and max_lag (the compute streams).  Into page-locked memory the
