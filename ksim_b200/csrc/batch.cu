@@ -441,6 +441,7 @@ ksim_status ksim_batch_create(const ksim_batch_job *jobs, int32_t n_jobs, const 
         double bytes = 0;
         for (const GraphDir &gd : c->img.gdir) bytes += (double)gd.stream_bytes + 64.0;
         const int64_t tile = k.sliced ? slice_shots(c) : (int64_t)k.threads * shots_per_thread(d.W);
+        if (k.sliced && !slice_tile_ok(4, (int)tile, 256)) return fail(KSIM_ERR_INTERNAL, "sliced tile width");
         if (k.sliced) k.ring_off = std::max(k.ring_off, slice_ring_off(c->slice_rows, c->slice_planes, (int)tile));
         for (int64_t s0 = 0; s0 < jb.B; s0 += tile) {
             BatchItem it = {};

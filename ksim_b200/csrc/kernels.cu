@@ -136,7 +136,7 @@ template <int S, int THREADS, int CTAS, int EVAL>
 cudaError_t launch_slice_as(const SampleJob &j, int shots, int threads, int tile, cudaStream_t st)
 {
     const int64_t blocks = (j.B + tile - 1) / tile;
-    if (blocks > 0x7FFFFFFF) return cudaErrorInvalidConfiguration;
+    if (blocks > 0x7FFFFFFF || !slice_tile_ok(S, shots, threads) || tile > shots) return cudaErrorInvalidConfiguration;
     const int smem = slice_smem_bytes(j.s_rows, j.s_planes, shots);
     cudaError_t e = cudaFuncSetAttribute(k_slice<S, THREADS, CTAS, EVAL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          SLICE_SMEM_MAX);

@@ -370,6 +370,7 @@ ksim_status admit(ksim_server *s, ServeRequest *r)
     // ones, which cost least a shot
     const int64_t by_shots = r->B <= 128 ? 128 : r->B <= 1024 ? 256 : r->B <= 8192 ? 512 : SERVE_SHOTS;
     const int64_t tile = s->cfg.threads > 0 ? std::min<int64_t>(by_shots, 4 * s->cfg.threads) : by_shots;
+    if (!slice_tile_ok(4, (int)tile, SERVE_THREADS)) return fail(KSIM_ERR_INTERNAL, "sliced tile width");
     std::vector<int> new_jobs;
     for (size_t k = 0; k < p->parts.size(); ++k) {
         ksim_component *c = p->parts[k].comp;

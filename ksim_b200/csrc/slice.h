@@ -56,6 +56,16 @@ constexpr int SLICE_AHEAD = 2;        // chunks staged at once
 // the bound it pays: 200,000 shots of those take 31 ms, from the records 115.
 constexpr size_t SLICE_MAX_BYTES = (size_t)1 << 30;
 
+// Tile widths slice_tile takes: a power of two up to the rows' 1,024 shots, whole
+// warps of S shots a lane (a lane without a shot of the tile would look up
+// result bytes that nothing wrote) and no more threads than the CTA has; S = 8
+// comes with two regions of rows.
+constexpr bool slice_tile_ok(int S, int shots, int threads)
+{
+    return (shots & (shots - 1)) == 0 && shots >= 64 && shots >= 32 * S && shots <= S * threads &&
+           (S == 8 ? shots == 2048 : shots <= 1024);
+}
+
 // A chunk has two parts, staged by copies of their own: the rows (this head,
 // its terms' SliceTerm, group lists and groups) and, behind them, the tables
 // (SliceValue, then look-up tables and value tables).  The head says what a

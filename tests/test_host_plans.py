@@ -1,6 +1,7 @@
 """Host plans, on the CPU: the item costs of a batch (ksim_b200/csrc/batch_plan.h:
 sliced and term-record items in one unit, so that kernels are ordered by time)
-and the chunks of a host call over sliced kernels (hostio.h)."""
+and the chunks of a host call over sliced kernels (hostio.h), and the widths of sliced
+tiles (slice.h)."""
 from __future__ import annotations
 
 import ctypes
@@ -76,3 +77,13 @@ def test_which_plan(emu):
         got, want = _bounds(emu, B, in_row, out_row, terms, graphs), _ramp(emu, B, in_row + out_row)
         assert (got == want) == ramp or len(want) == 2, (B, in_row, out_row, terms)
         assert _bounds(emu, B, in_row, out_row, terms, graphs, sliced=0) == want
+
+
+def test_tile_widths(emu):
+    """The widths the launches choose pass; those a warp of lanes would not fill,
+    or a CTA would not cover, are refused on the host."""
+    ok = [(1, 128, 512), (1, 256, 512), (1, 512, 512), (4, 1024, 512), (4, 1024, 256), (8, 2048, 256),
+          *((4, 4 * t, t) for t in (32, 64, 128, 256)), *((4, n, 256) for n in (128, 256, 512))]
+    bad = [(4, 64, 256), (4, 32, 256), (4, 96, 256), (4, 192, 256), (4, 2048, 512), (4, 512, 64), (8, 1024, 256),
+           (8, 4096, 512), (1, 32, 512), (1, 1024, 512), (1, 0, 512)]
+    assert [x for x in ok if not emu.plan_tile_ok(*x)] == [] and [x for x in bad if emu.plan_tile_ok(*x)] == []
