@@ -168,3 +168,19 @@ def test_stream_size_bound(emu):
     full = f(descs, 3, 10, 1 << 30)
     assert info(emu, gs, 10)["big"] == 18 and full == info(emu, gs, 10)["bytes"] > 18 * 16384
     assert f(descs, 3, 10, full) == full and f(descs, 3, 10, full - 16384) == 0 and f(descs, 3, 10, 0) == 0
+
+
+@pytest.mark.parametrize("kind", ["narrow", "hybrid", "all"])
+@pytest.mark.parametrize("F", [20, 100, 160, 240])
+def test_components_kept_on_term_records(emu, kind, F):
+    """The components the GPU tests of the term-record kernels use have no sliced
+    stream, and the term paths they are named for; the same graphs without the
+    scaled-down term have one."""
+    import unsliced
+    from ksim_b200.perfmodel import component_work
+    comp = unsliced.component(kind, F)
+    w = component_work(comp)
+    paths = [w["hybrid_terms"] > 0, w["wide_terms"] + w["exact_terms"] > 0]
+    assert paths == {"narrow": [False, False], "hybrid": [True, False], "all": [True, True]}[kind]
+    assert not info(emu, comp.graphs, F)["ok"]
+    assert info(emu, unsliced.component(kind, F, sliced=True).graphs, F)["ok"]
