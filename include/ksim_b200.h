@@ -113,6 +113,9 @@ int32_t ksim_component_num_f(const ksim_component *c);
 int32_t ksim_component_n_graphs(const ksim_component *c);
 int32_t ksim_component_words(const ksim_component *c);   /* 64-bit words per parameter vector */
 int64_t ksim_component_image_bytes(const ksim_component *c);
+/* 1 if the component has a sliced stream (its terms as sign counts and value
+ * tables, sampled 64 shots a lane), 0 if its kernels run the term records. */
+int32_t ksim_component_sliced(const ksim_component *c);
 
 /* Host buffers, synchronous.  f_sel: (B, num_f) uint8 C-contiguous; out:
  * (B, max(n_out,1)) uint8.  Replaces Component.sample, kokkos_sim.cpp:188-241

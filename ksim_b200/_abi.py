@@ -195,6 +195,7 @@ def _declare(L: ctypes.CDLL) -> None:
         "ksim_component_n_graphs": (i32, [vp]),
         "ksim_component_words": (i32, [vp]),
         "ksim_component_image_bytes": (i64, [vp]),
+        "ksim_component_sliced": (i32, [vp]),
         "ksim_component_sample": (i32, [vp, _u8p, i64, u64, i32, _u8p]),
         "ksim_component_sample_device": (i32, [vp, vp, i64, i64, u64, i32, vp, i64, i64,
                                                vp, vp]),

@@ -13,8 +13,8 @@ with the same seed — shot s of a job always uses stream index s, whatever
 else shares the launch.
 
 ``tune()`` is the autotuner: it times a small grid of launch shapes (shots
-per work item, staging slot size, persistent CTAs per SM) on the batch
-itself and keeps the fastest; results are cached per GPU and batch shape in
+per work item, staging slot size, persistent CTAs per SM; those that differ
+for the batch's jobs) on the batch itself and keeps the fastest; results are cached per GPU and batch shape in
 ``$KSIM_B200_TUNE_CACHE`` (default ``~/.cache/ksim_b200/tuning.json``).
 """
 from __future__ import annotations
@@ -39,6 +39,20 @@ _CANDIDATES = [
     {"threads": t, "slot_bytes": s, "ctas_per_sm": c}
     for t in (64, 128, 256) for s in (8192, 12288, 14336, 16384) for c in (0, 4)
 ]
+
+
+def _shapes(sliced: bool) -> list:
+    """The launch shapes tune() tries.  Sliced jobs have CTAs of 256 threads and
+    slots of their own: of the grid only threads <= 64 (tiles of at most 512
+    shots) changes their items and ctas_per_sm, up to the two an SM holds, their
+    CTAs, so without term-record jobs one shape of each kind is timed (the one
+    with the largest slot, which a job's largest term must still fit)."""
+    if not sliced:
+        return _CANDIDATES
+    kinds: dict = {}
+    for c in sorted(_CANDIDATES, key=lambda c: -c["slot_bytes"]):
+        kinds.setdefault((c["threads"] <= 64, min(c["ctas_per_sm"] or 2, 2)), c)
+    return list(kinds.values())
 
 
 def tune_cache_path() -> Path:
@@ -233,7 +247,8 @@ class BatchSampler:
                 return hit
         max_term = max(kc.stats()["max_term_bytes"] for s in self.samplers for _, kc in s.components)
         results = []
-        for cand in (candidates or _CANDIDATES):
+        sliced = all(kc.sliced for s in self.samplers for _, kc in s.components if kc.n_out)
+        for cand in (candidates or _shapes(sliced)):
             if cand["slot_bytes"] < max_term:
                 continue
             try:

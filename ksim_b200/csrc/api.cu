@@ -289,6 +289,7 @@ int32_t ksim_component_num_f(const ksim_component *c) { return c ? c->img.F : -1
 int32_t ksim_component_n_graphs(const ksim_component *c) { return c ? c->img.n_graphs : -1; }
 int32_t ksim_component_words(const ksim_component *c) { return c ? c->img.W : -1; }
 int64_t ksim_component_image_bytes(const ksim_component *c) { return c ? (int64_t)c->image_bytes : -1; }
+int32_t ksim_component_sliced(const ksim_component *c) { return c ? (c->d_slices ? 1 : 0) : -1; }
 
 ksim_status ksim_component_set_launch(ksim_component *c, int32_t threads, int32_t staged, int32_t slot_bytes)
 {

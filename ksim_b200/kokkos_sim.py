@@ -88,6 +88,12 @@ class Component:
         """64-bit words per parameter vector in the device image."""
         return int(self._L.ksim_component_words(self._h))
 
+    @property
+    def sliced(self) -> bool:
+        """Whether the component has a sliced stream (else its kernels run the
+        term records)."""
+        return self._L.ksim_component_sliced(self._h) == 1
+
     def sample(self, f_sel, seed, rng_mode: int = RNG_XORSHIFT) -> np.ndarray:
         f = _rows_u8(f_sel, "f_sel")
         if f.shape[1] != self._num_f:

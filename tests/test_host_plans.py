@@ -87,3 +87,11 @@ def test_tile_widths(emu):
     bad = [(4, 64, 256), (4, 32, 256), (4, 96, 256), (4, 192, 256), (4, 2048, 512), (4, 512, 64), (8, 1024, 256),
            (8, 4096, 512), (1, 32, 512), (1, 1024, 512), (1, 0, 512)]
     assert [x for x in ok if not emu.plan_tile_ok(*x)] == [] and [x for x in bad if emu.plan_tile_ok(*x)] == []
+
+
+def test_tuner_shapes():
+    """Without term-record jobs the autotuner times each distinct shape once."""
+    from ksim_b200.batch import _CANDIDATES, _shapes
+    assert _shapes(False) == _CANDIDATES
+    got = [(c["threads"] <= 64, c["slot_bytes"]) for c in _shapes(True)]
+    assert sorted(got) == [(False, 16384), (True, 16384)]
