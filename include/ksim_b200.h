@@ -186,7 +186,13 @@ ksim_status ksim_component_status(ksim_component *c, uint32_t *flags, int32_t re
 /* Launch shape of the plain sampler for this component: threads per CTA
  * (a multiple of 32, <= 256), whether term chunks are staged in shared memory
  * by TMA bulk copies, and the staging slot size in bytes (>= the largest term
- * record, a multiple of 16).  Zero / negative values keep the current value. */
+ * record, a multiple of 16).  Zero / negative values keep the current value.
+ * That is the shape of the term-record kernels.  A component with a sliced
+ * stream (ksim_component_sliced) takes its tile shape from the shots of a call;
+ * once threads is given, tiles of 4 x threads shots by CTAs of that many
+ * threads, rounded down to 32, 64, 128 or 256.  staged and slot_bytes are
+ * checked and kept for it too, but only the allocation-free entry point, which
+ * runs the term records, uses them. */
 ksim_status ksim_component_set_launch(ksim_component *c, int32_t threads, int32_t staged,
                                       int32_t slot_bytes);
 ksim_status ksim_component_get_launch(const ksim_component *c, int32_t *threads, int32_t *staged,
@@ -301,16 +307,21 @@ typedef struct ksim_batch_job {
 } ksim_batch_job;
 
 /* Launch shape of a batch (zero / negative fields take the defaults:
- * 128 threads, 14 KiB slots, CTAs per SM from occupancy, graph on).  The
- * shape applies to the jobs whose terms all run on 32-bit words with W <= 4
- * (the bulk of the work), drained by one persistent kernel; jobs with hybrid,
+ * 128 threads, 14 KiB slots, CTAs per SM from occupancy, graph on).
+ * Jobs with a sliced stream (ksim_component_sliced) run one body: items of
+ * 256, 512 or 1,024 shots by the job's share of the batch (at most 512 if
+ * threads <= 64), CTAs of 256 threads with slots of their own, all of them
+ * drawing from one list, ctas_per_sm of them an SM.
+ * Of the other jobs the shape applies to those whose terms all run on 32-bit
+ * words with W <= 4, drained by one persistent kernel a W; jobs with hybrid,
  * 64-bit or exact-path terms and jobs with W > 4 run in kernels of their own
  * (CTAs of 128; slots of at least 16 KiB for 64-bit, exact and W > 4 terms),
- * launched before it and overlapping it.  A work item is 2 x threads shots of a W <= 4 job
- * (two shots per thread) and threads shots of a wider one. */
+ * launched before it and overlapping it.  Their work item is 2 x threads shots
+ * of a W <= 4 job (two shots per thread) and threads shots of a wider one. */
 typedef struct ksim_batch_tuning {
     int32_t threads;      /* threads per CTA (a multiple of 32, <= 256); see the item size above */
-    int32_t slot_bytes;   /* staging slot, multiple of 16, >= the largest term of every 32-bit job */
+    int32_t slot_bytes;   /* staging slot, multiple of 16, >= the largest term of every job whose
+                             terms all run on 32-bit words (sliced jobs are held to it too) */
     int32_t ctas_per_sm;  /* persistent CTAs per SM (<= occupancy limit) */
     int32_t use_graph;    /* 1: capture counter reset + kernels in a CUDA graph */
 } ksim_batch_tuning;
@@ -355,8 +366,13 @@ typedef struct ksim_server_config {
     int64_t arena_bytes;     /* admission budget for request buffers (default 1 GiB) */
     int32_t max_requests;    /* request slots in flight (default 1024)               */
     int32_t max_jobs;        /* job-table slots in flight (default 4096)             */
-    int32_t threads;         /* shots per tile = threads per CTA (default 128)       */
-    int32_t slot_bytes;      /* staging slot of the loop kernel (default 16 KiB)     */
+    int32_t threads;         /* a multiple of 32, <= 256: sliced tiles of at most
+                                4 x threads shots, rounded down to a power of two
+                                (default: by the request's shots, 128 to 1,024); the
+                                loop's CTAs have 256 threads, its term-record tiles
+                                512 shots                                            */
+    int32_t slot_bytes;      /* staging slot of term-record tiles (default 16 KiB;
+                                at most 24 KiB of it are used)                       */
     int32_t ctas_per_sm;     /* loop CTAs per SM (default: occupancy limit)          */
     int32_t idle_us;         /* the loop exits after the whole grid claimed no work
                                 for this long (default 2000)                         */

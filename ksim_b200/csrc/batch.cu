@@ -161,8 +161,7 @@ __global__ void __launch_bounds__(256, 2) k_batch_s(const __grid_constant__ PT P
 {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ int s_item;
-    uint8_t *ring = smem + P.slot_bytes;
-    uint64_t *bar = (uint64_t *)ring;
+    uint64_t *bar = (uint64_t *)(smem + P.slot_bytes);
     slice_ring_init(bar);
     pdl_launch_dependents();
     uint32_t g = 0;
@@ -175,7 +174,7 @@ __global__ void __launch_bounds__(256, 2) k_batch_s(const __grid_constant__ PT P
         const BatchItem w = P.items[it];
         const SampleJob &j = P.job(w.job).j;
         const int64_t end = w.s0 + w.shots < j.B ? w.s0 + w.shots : j.B;
-        if (!slice_tile<4>(j, w.s0, end, w.shots, smem, slice_rows_bytes(j.s_rows, w.shots), bar, ring + BAR_BYTES, g))
+        if (!slice_tile<4>(j, w.s0, end, w.shots, smem, slice_rows_bytes(j.s_rows, w.shots), bar, g))
             break;
     }
     pdl_wait();

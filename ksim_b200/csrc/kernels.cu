@@ -51,8 +51,8 @@ __global__ void __launch_bounds__(THREADS, CTAS) k_slice(const SampleJob j, cons
     slice_ring_init(bar);
     uint32_t g = 0;
     const int64_t s0 = (int64_t)blockIdx.x * tile;
-    slice_tile<S, false, EVAL>(j, s0, s0 + tile < j.B ? s0 + tile : j.B, shots, smem, slice_rows_bytes(j.s_rows, shots), bar,
-                  ring + BAR_BYTES, g);
+    slice_tile<S, false, EVAL>(j, s0, s0 + tile < j.B ? s0 + tile : j.B, shots, smem,
+                               slice_rows_bytes(j.s_rows, shots), bar, g);
 }
 
 template <int W>
@@ -163,7 +163,7 @@ cudaError_t launch_slice_as(const SampleJob &j, int shots, int threads, int tile
 template <int EVAL = -1>
 cudaError_t launch_slice(const SampleJob &j, const LaunchCfg &cfg, cudaStream_t st)
 {
-    if (cfg.slice_threads > 0) {  // threads chosen by the caller: four shots each
+    if (cfg.slice_threads > 0) {  // chosen by the caller: four shots each, a power of two of threads
         const int t = cfg.slice_threads >= 256 ? 256 : cfg.slice_threads >= 128 ? 128 : cfg.slice_threads >= 64 ? 64 : 32;
         return launch_slice_as<4, 256, 2, EVAL>(j, 4 * t, t, 4 * t, st);
     }

@@ -25,9 +25,9 @@
 // issued and returns false without writing outputs.
 //
 // CG = true reads every job-dependent array (directories, f rows, column
-// maps) with L2-only loads.  The serving loop (which runs the
-// sliced tile) needs that: its CTAs live across requests, and a request's buffers may reuse memory an earlier
-// request of the same kernel lifetime read through this SM's L1.
+// maps) with L2-only loads.  The serving loop needs that: its CTAs live across
+// requests, and a request's buffers may reuse memory an earlier request of the
+// same kernel lifetime read through this SM's L1.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(SERVE_THREADS, 2) k_serve(ServeJob *jobs, Serv
             uint8_t *slots = smem + SERVE_RING + BAR_BYTES;
             const bool ok =
                 s_W == 0 ? slice_tile<4, true>(s_job, s0, s0 + shots < s_job.B ? s0 + shots : s_job.B, shots, smem,
-                                               slice_rows_bytes(s_job.s_rows, shots), bar, slots, g)
+                                               slice_rows_bytes(s_job.s_rows, shots), bar, g)
                          : serve_record_tile(s_W, s_paths, s_job, s0, record_bar, slots, record_g, smem);
             __threadfence();  // this thread's outputs before the counters below
             __syncthreads();

@@ -101,9 +101,8 @@ void cast(const El &x, int64_t p2, double &re, double &im)
     }
 }
 
-// A parity row: its parameters (one bit each) and whether its parity is
-// complemented.  (As lists of indices, allocated a row, a 64-program
-// pool took 0.26 s to build, now 0.18.)
+// A parity row: its parameters (one bit each, so that nothing is allocated a
+// row) and whether its parity is complemented.
 struct Row {
     uint64_t bits[4] = {0, 0, 0, 0};
     uint32_t inv = 0;
@@ -225,9 +224,9 @@ struct TermRows {
     }
 };
 
-// A group of SLICE_GROUP rows of one role: 4 bytes a row of complement masks, then index units: four
-// slots of each row (a byte is a parameter row; the rows with fewer name the
-// zero row).
+// A group of SLICE_GROUP rows of one role: 4 bytes a row of complement masks,
+// then index units: four slots of each row (a byte is a parameter row; the rows
+// with fewer name the zero row).
 struct Group {
     std::vector<uint8_t> bytes;
     uint32_t slots = 0;  // index slots a row

@@ -98,8 +98,9 @@ enum : uint32_t { ST_WIDE = 1u, ST_BIG = 2u, ST_EVEN = 4u };
 // pairs, into S; kill.
 enum { SQ_W1, SQ_W2, SQ_W4, SQ_N9, SQ_PPK, SQ_X1, SQ_X0, SQ_PPX, SQ_KILL, SQ_ROLES };
 
-// One term of a chunk, in either part.  Its rows come in groups of four, listed role by role as u32: bits 0-15 the group's offset in the chunk /
-// 16, 16-23 its index slots a row, 24-27 the role.
+// One term of a chunk, in either part.  Its rows come in groups of four, listed
+// role by role as u32: bits 0-15 the group's offset in the chunk / 16, 16-23 its
+// index slots a row, 24-27 the role.
 constexpr int SLICE_GROUP = 4;
 struct SliceTerm {
     uint16_t list_off16;  // group list (16-byte units, in the rows part)

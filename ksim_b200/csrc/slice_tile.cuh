@@ -456,15 +456,14 @@ __device__ __forceinline__ uint2 lds64(uint32_t a)
 }
 
 // Sample shots [s0, s_end) of job j in a tile of `shots`, S of them a thread
-// (shots / S threads, whole warps: a lane without a shot of the tile would look
-// up result bytes that nothing wrote; the others only share the rows pass).  smem: the CTA's shared
-// memory, parameter rows first, planes at planes_off.  Returns false after a
-// wait timeout (the CTA must then stop using the ring).
+// (slice_tile_ok; threads past shots / S only share the rows pass).  smem: the
+// CTA's shared memory, parameter rows first, planes at planes_off.  Returns
+// false after a wait timeout (the CTA must then stop using the ring).
 // EVAL: instead of sampling, the job's chunks are one graph's and its rows are
 // whole parameter vectors; |A| (EVAL_ABS) or A (EVAL_COMPLEX) goes to j.amp.
 template <int S, bool CG = false, int EVAL = -1>
 __device__ __forceinline__ bool slice_tile(const SampleJob &j, const int64_t s0, const int64_t s_end, int shots,
-                                           uint8_t *smem, int planes_off, uint64_t *bar, uint8_t *, uint32_t &g)
+                                           uint8_t *smem, int planes_off, uint64_t *bar, uint32_t &g)
 {
     uint8_t *slots = (uint8_t *)bar + BAR_BYTES;
     static_assert(S == 1 || S == 4 || S == 8, "shots per thread");
