@@ -73,12 +73,12 @@ NCU_DRAM_BYTES_PER_SHOT = {"cfg2-medium-40q-t12": 65.2 + 40.0, "cfg4-large-rank-
 # the SMs' issue ceiling (capture command and figures: the ncu summaries
 # under profiles/).
 NCU_THREAD_INST_PER_SHOT = {"cfg2-medium-40q-t12": 27464, "cfg4-large-rank-85q-t20": 32099}
-# Thread instructions of one cfg3 batch (its five class kernels, one ncu
-# capture at the default launch shape: 128 threads, 14 KiB slots); the
-# batched leg's issue fraction is this over its timed batch and the issue
-# ceiling (capture command and figures: the ncu summaries under profiles/).
+# Thread instructions of one cfg3 batch (the launch of k_batch_s that has the
+# CTAs, one ncu capture at the default launch shape; its jobs are all sliced, so
+# threads above 64 and the slot size change nothing); the batched leg's issue
+# fraction is this over its timed batch and the issue ceiling (capture command
+# and figures: the ncu summaries under profiles/).
 NCU_THREAD_INST_PER_BATCH = 17.88e9
-NCU_BATCH_SHAPE = {"threads": 128, "slot_bytes": 14336, "ctas_per_sm": 0}
 # Gate locations of the workloads' circuits (qubits x depth): one
 # single-qubit Pauli channel each in the noisy end-to-end leg.
 NOISE_LOCATIONS = {"cfg2-medium-40q-t12": 40 * 200, "cfg4-large-rank-85q-t20": 85 * 600}
@@ -448,9 +448,9 @@ def bench_batched(args, torch, dev, flush):
             "plain_launches": len(ws), "tuning": rec["tuning"], "work_items": info["items"],
             "grid": info["grid"],
             "issue_frac": NCU_THREAD_INST_PER_BATCH / (mb / 1e3) / issue_ceiling(torch, dev),
-            "issue_note": "ncu thread instructions of one batch at the launch shape "
-                          f"{NCU_BATCH_SHAPE} (this run: {rec['tuning']}) over the timed batch and "
-                          "148 SMs x 4 x 32 lanes x 1965 MHz"}
+            "issue_note": "ncu thread instructions of one batch with tiles of up to 1,024 shots and two "
+                          f"CTAs an SM, whatever the slot size (this run: {rec['tuning']}), over the timed "
+                          "batch and 148 SMs x 4 x 32 lanes x 1965 MHz"}
 
 
 class _PinnedRing:
@@ -587,6 +587,14 @@ def bench_served(args, torch, dev):
     lat = np.array(done) - (t0 + arrivals)
     served = float(shots.sum()) / (max(done) - t0)
     st = srv.stats()
+    # the same requests at that fraction of the served capacity: a load the
+    # server carries, where the latencies are not queue lengths
+    carried_rate = args.load * capacity / float(shots.mean())
+    carried_arrivals = np.cumsum(rng.exponential(1.0 / carried_rate, n_req))
+    ct0, cdone = _replay(carried_arrivals, submit, collect)
+    clat = np.array(cdone) - (ct0 + carried_arrivals)
+    carried = float(shots.sum()) / (max(cdone) - ct0)
+    carried_failed = srv.stats()["failed"] - st["failed"]
     srv.close()
 
     # the same stream through plain per-request calls, in arrival order
@@ -617,6 +625,9 @@ def bench_served(args, torch, dev):
             "load_basis": "batched capacity of the request mix (first requests as one batch)",
             "batched_capacity_shots_per_s": batched_capacity, "batched_tuning": batched_tuning,
             "served_capacity_shots_per_s": capacity,
+            "at_served_capacity": {"load": args.load, "load_basis": "served capacity (a closed burst)",
+                                   "arrival_rate_per_s": carried_rate, "shots_per_s": carried,
+                                   "p50_ms": q(clat, 50), "p99_ms": q(clat, 99), "failed": carried_failed},
             "total_shots": int(shots.sum()),
             "loop_launches": st["loop_launches"] - before["loop_launches"],
             "failed": st["failed"], "clock": "host wall clock, arrival -> results in host memory"}
@@ -785,7 +796,8 @@ def main():
                            f"({sm_mhz:.0f} MHz)",
             "ops_per_shot": work["ops"],
             "ops_per_shot_reference_model": ref_ops,
-            "ops_note": "ops_per_shot: int32 operations of the formulation the kernels run; "
+            "ops_note": "ops_per_shot: int32 operations of the term-record kernels' formulation (the sliced "
+                        "kernel does the same shots with fewer, so fractions of that model pass 1); "
                         "ops_per_shot_reference_model: the reference's step-by-step algorithm "
                         "(84 per Z[w] product, 5 per 64-bit parity word); neither is an issue count",
             "int_ops_per_s": achieved,
