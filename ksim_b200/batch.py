@@ -4,11 +4,10 @@
 input buffer (the full f matrix) and one device output buffer per program,
 and turns every component of every program into a job of one
 ``ksim_batch`` (``include/ksim_b200.h``): longest-first work items pulled by
-persistent CTAs, one kernel per (W, term paths) class of jobs, the class
-kernels chained on one stream as programmatic dependent launches (each
-starts while the one before it drains), all captured in a CUDA graph and
-replayed.  Each
-program's result is bit-identical to ``B200ProgramSampler(prog).sample``
+persistent CTAs, one body and one list for all jobs with a sliced stream, one
+kernel per (W, term paths) class of the others, the kernels chained on one
+stream as programmatic dependent launches (each starts while the one before it
+drains), all captured in a CUDA graph and replayed.  Each program's result is bit-identical to ``B200ProgramSampler(prog).sample``
 with the same seed — shot s of a job always uses stream index s, whatever
 else shares the launch.
 

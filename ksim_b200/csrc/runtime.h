@@ -88,7 +88,8 @@ struct ksim_program {
     std::vector<cudaEvent_t> ev_in, ev_done;  // per chunk, kept across calls
     uint32_t *h_status = nullptr;             // page-locked: the components' status words after a call
     int64_t sms = 1;                          // SMs of the device
-    int64_t wave_shots = 1;                   // shots one wave of sampling CTAs holds on the device
+    int64_t wave_shots = 1;                   // shots one wave of term-record CTAs holds on the device (the
+                                              // copy lag's measure; sliced calls keep the same lag)
     ksim::DevBuf ws_f, ws_out, ws_fp, ws_op;  // unpacked rows; bit-packed rows
     std::mutex mu;
 };
