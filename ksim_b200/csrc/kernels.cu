@@ -160,6 +160,11 @@ cudaError_t launch_slice_as(const SampleJob &j, int shots, int threads, int tile
 // but a narrower one that still fits one wave ends sooner.  Two CTAs of 2,048
 // shots need at most 129 parameter rows; with more (60 outputs, F = 100) one
 // CTA took 1.318 ms for 606,208 shots, two of 1,024 take 1.002.
+// Chunks of at most four terms (eight planes) have work for eight warps in the
+// rows pass, and sixteen only wait for one another: with 256 threads 80,000 shots
+// of a program of one term a graph and 5, 20, 60 outputs take 24.8, 72.6, 199 us
+// (512: 26.2, 75.9, 205), 5,000 shots 16.6, 49.3, 127 (16.8, 50.2, 131); of eight
+// terms a graph and 3 outputs 5,000 shots 20.6 (18.6).
 template <int EVAL = -1>
 cudaError_t launch_slice(const SampleJob &j, const LaunchCfg &cfg, cudaStream_t st)
 {
@@ -171,11 +176,15 @@ cudaError_t launch_slice(const SampleJob &j, const LaunchCfg &cfg, cudaStream_t 
     // (launches of one call overlap: their shape is that of the call's shots, up
     // to the two-per-SM width, which the launches in flight fill together)
     const int64_t n = cfg.call_shots > 0 ? std::min(cfg.call_shots, 2 * sms * 1024) : j.B;
+    const bool few = j.s_planes <= 8;
     if (n <= sms * 512) {
         const int shots = n <= sms * 128 ? 128 : n <= sms * 256 ? 256 : 512;
-        return launch_slice_as<1, 512, 1, EVAL>(j, shots, 512, shots, st);
+        return launch_slice_as<1, 512, 1, EVAL>(j, shots, few && shots <= 256 ? 256 : 512, shots, st);
     }
-    if (n <= sms * 1024) return launch_slice_as<4, 512, 1, EVAL>(j, 1024, 512, 1024, st);
+    if (n <= sms * 1024) {
+        if (few) return launch_slice_as<4, 256, 2, EVAL>(j, 1024, 256, 1024, st);
+        return launch_slice_as<4, 512, 1, EVAL>(j, 1024, 512, 1024, st);
+    }
     const bool wide = n > 2 * sms * 1024 && slice_two_ctas(j.s_rows, j.s_planes, 2048);
     const int shots = wide ? 2048 : 1024;
     // equal tiles: a last wave that is nearly empty costs as much as a full one

@@ -105,3 +105,22 @@ def test_non_finite_approximation_factor(cuda_device, oracle_port):
     got = kc.eval_abs(2, pv)
     nan = np.isnan(a).any(1)
     assert np.array_equal(np.isnan(got), nan) and np.array_equal(np.isinf(got), np.isinf(a).any(1) & ~nan)
+
+
+@pytest.mark.parametrize("G", [4, 5])
+def test_tile_shapes_by_terms(cuda_device, oracle_port, G):
+    """The shot counts around the launch rule's lines for components with chunks
+    of at most four terms, and of more (CTAs of 256 and of 512 threads)."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    rng, graphs = _graphs(40 + G, 16, 3, G=G)
+    f = rng.integers(0, 2, size=(sms * 1024 + 1, 16)).astype(np.uint8)
+    want, want_amp = oracle_port.PortOracle(graphs, 16).sample(f, 9, 0, return_amp=True)
+    kc = _component(graphs, 16)
+    for edge in (1, 128, sms * 128, sms * 256, sms * 512, sms * 1024):
+        for B in (edge, edge + 1):
+            bits, amp = device_sample(kc, f[:B], 9, 0)
+            assert np.array_equal(bits, want[:B]) and same_bits(amp, want_amp[:B]), B
+    pv = rng.integers(0, 2, size=(sms * 1024, 18)).astype(np.uint8)
+    for B in (100, sms * 256, sms * 512, sms * 1024):
+        assert same_bits(kc.eval_abs(2, pv[:B]), oracle_port.PortOracle(graphs, 16).eval_abs(2, pv[:B])), B
