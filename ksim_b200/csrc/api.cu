@@ -89,11 +89,6 @@ ksim_status component_chunks(ksim_component *c, int slot_bytes, const ChunkDir *
     return KSIM_OK;
 }
 
-static ksim_status fail_timeout()
-{
-    return fail(KSIM_ERR_TIMEOUT, "a staging wait of the sampling kernel ran out; its shots were not written");
-}
-
 // A component's status word as read after a call (`flags`): a wait that
 // ran out fails the call and is cleared from the word (the other flags stay
 // for ksim_component_status).
@@ -103,7 +98,15 @@ ksim_status report_timeout_flags(ksim_component *c, uint32_t flags)
     const uint32_t rest = flags & ~(uint32_t)KSIM_FLAG_WAIT_TIMEOUT;
     const cudaError_t e = cudaMemcpy(c->d_status, &rest, sizeof(rest), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cuda_fail(e, "status write");
-    return fail_timeout();
+    return fail(KSIM_ERR_TIMEOUT, "a staging wait of the sampling kernel ran out; its shots were not written");
+}
+
+ksim_status report_timeout(ksim_component *c)
+{
+    uint32_t flags = 0;
+    cudaError_t e = cudaMemcpy(&flags, c->d_status, sizeof(flags), cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) return cuda_fail(e, "status read");
+    return report_timeout_flags(c, flags | KSIM_FLAG_WAIT_TIMEOUT);
 }
 
 // Fill a SampleJob for component c; inputs/outputs set by the caller.
@@ -238,10 +241,6 @@ ksim_status ksim_component_create(const ksim_graph_desc *graphs, int32_t n_graph
     if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(status)");
     e = cudaMemset(c->d_status, 0, sizeof(uint32_t));
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemset(status)");
-    // (here and not in the first eval call: a process's first page-locked
-    // allocation takes over a millisecond, later ones some microseconds)
-    e = cudaMallocHost(&c->h_status, sizeof(uint32_t));
-    if (e != cudaSuccess) return cuda_fail(e, "cudaMallocHost(status)");
     e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamCreate");
     // default launch shape: slot fits the largest term and at least 16 KiB;
@@ -276,7 +275,6 @@ void ksim_component_destroy(ksim_component *c)
     c->ws_out.release();
     c->ws_aux.release();
     if (c->d_status) cudaFree(c->d_status);
-    if (c->h_status) cudaFreeHost(c->h_status);
     if (c->d_image) cudaFree(c->d_image);
     if (c->d_slices) cudaFree(c->d_slices);
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -463,20 +461,23 @@ static ksim_status eval_common(ksim_component *c, int32_t graph, const uint8_t *
         s.f_stride = P;
         s.amp = (double *)c->ws_aux.p;
         s.B = B;
-        // this kernel stages chunks: a wait that ran out left rows unwritten.  Its
-        // one flag goes to a page-locked word (copying the component's back took
-        // 3.6 us of a 43 us call, 9 of a 340 us one), the component's stays as it is
-        volatile uint32_t *flags = c->h_status;
-        *flags = 0;
-        s.status = c->h_status;
+        s.status = c->d_status;
         s.wait_limit = c->wait_limit;
-        e = launch_eval_sliced(s, mode, cfg, c->stream);
+        int tile = 1;
+        e = launch_eval_sliced(s, mode, cfg, c->stream, &tile);
         if (e != cudaSuccess) return cuda_fail(e, "eval kernel launch");
         e = cudaMemcpyAsync(out, c->ws_aux.p, out_bytes, cudaMemcpyDeviceToHost, c->stream);
         const cudaError_t end = cudaStreamSynchronize(c->stream);
         if (e == cudaSuccess) e = end;
         if (e != cudaSuccess) return cuda_fail(e, "eval");
-        return *flags & KSIM_FLAG_WAIT_TIMEOUT ? fail_timeout() : KSIM_OK;
+        // this kernel stages chunks: a tile whose wait ran out marked its first row
+        const size_t row_bytes = out_bytes / (size_t)B;
+        for (int64_t r = 0; r < B; r += tile) {
+            uint64_t v;
+            std::memcpy(&v, (const uint8_t *)out + (size_t)r * row_bytes, sizeof(v));
+            if (v == SLICE_UNWRITTEN) return report_timeout(c);
+        }
+        return KSIM_OK;
     }
     EvalJob j = {};
     j.image = c->d_image;

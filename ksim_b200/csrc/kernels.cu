@@ -133,8 +133,9 @@ cudaError_t launch_sample_w(const SampleJob &j, const LaunchCfg &cfg, cudaStream
 }
 
 template <int S, int THREADS, int CTAS, int EVAL>
-cudaError_t launch_slice_as(const SampleJob &j, int shots, int threads, int tile, cudaStream_t st)
+cudaError_t launch_slice_as(const SampleJob &j, int shots, int threads, int tile, cudaStream_t st, int *tile_used)
 {
+    if (tile_used) *tile_used = tile;
     const int64_t blocks = (j.B + tile - 1) / tile;
     if (blocks > 0x7FFFFFFF || !slice_tile_ok(S, shots, threads) || tile > shots) return cudaErrorInvalidConfiguration;
     const int smem = slice_smem_bytes(j.s_rows, j.s_planes, shots);
@@ -166,11 +167,11 @@ cudaError_t launch_slice_as(const SampleJob &j, int shots, int threads, int tile
 // (512: 26.2, 75.9, 205), 5,000 shots 16.6, 49.3, 127 (16.8, 50.2, 131); of eight
 // terms a graph and 3 outputs 5,000 shots 20.6 (18.6).
 template <int EVAL = -1>
-cudaError_t launch_slice(const SampleJob &j, const LaunchCfg &cfg, cudaStream_t st)
+cudaError_t launch_slice(const SampleJob &j, const LaunchCfg &cfg, cudaStream_t st, int *tile_used = nullptr)
 {
     if (cfg.slice_threads > 0) {  // chosen by the caller: four shots each, a power of two of threads
         const int t = cfg.slice_threads >= 256 ? 256 : cfg.slice_threads >= 128 ? 128 : cfg.slice_threads >= 64 ? 64 : 32;
-        return launch_slice_as<4, 256, 2, EVAL>(j, 4 * t, t, 4 * t, st);
+        return launch_slice_as<4, 256, 2, EVAL>(j, 4 * t, t, 4 * t, st, tile_used);
     }
     const int64_t sms = cfg.sms;
     // (launches of one call overlap: their shape is that of the call's shots, up
@@ -179,11 +180,11 @@ cudaError_t launch_slice(const SampleJob &j, const LaunchCfg &cfg, cudaStream_t 
     const bool few = j.s_planes <= 8;
     if (n <= sms * 512) {
         const int shots = n <= sms * 128 ? 128 : n <= sms * 256 ? 256 : 512;
-        return launch_slice_as<1, 512, 1, EVAL>(j, shots, few && shots <= 256 ? 256 : 512, shots, st);
+        return launch_slice_as<1, 512, 1, EVAL>(j, shots, few && shots <= 256 ? 256 : 512, shots, st, tile_used);
     }
     if (n <= sms * 1024) {
-        if (few) return launch_slice_as<4, 256, 2, EVAL>(j, 1024, 256, 1024, st);
-        return launch_slice_as<4, 512, 1, EVAL>(j, 1024, 512, 1024, st);
+        if (few) return launch_slice_as<4, 256, 2, EVAL>(j, 1024, 256, 1024, st, tile_used);
+        return launch_slice_as<4, 512, 1, EVAL>(j, 1024, 512, 1024, st, tile_used);
     }
     const bool wide = n > 2 * sms * 1024 && slice_two_ctas(j.s_rows, j.s_planes, 2048);
     const int shots = wide ? 2048 : 1024;
@@ -192,8 +193,8 @@ cudaError_t launch_slice(const SampleJob &j, const LaunchCfg &cfg, cudaStream_t 
     const int64_t waves = (all + 2 * sms * shots - 1) / (2 * sms * shots);
     const int64_t want = (all + waves * 2 * sms - 1) / (waves * 2 * sms);
     const int tile = (int)((want + 63) / 64 * 64);
-    if (wide) return launch_slice_as<8, 256, 2, EVAL>(j, shots, 256, tile, st);
-    return launch_slice_as<4, 256, 2, EVAL>(j, shots, 256, tile, st);
+    if (wide) return launch_slice_as<8, 256, 2, EVAL>(j, shots, 256, tile, st, tile_used);
+    return launch_slice_as<4, 256, 2, EVAL>(j, shots, 256, tile, st, tile_used);
 }
 
 template <int W>
@@ -282,10 +283,11 @@ cudaError_t launch_sample(const SampleJob &job, int W, const LaunchCfg &cfg, cud
     }
 }
 
-cudaError_t launch_eval_sliced(const SampleJob &job, int mode, const LaunchCfg &cfg, cudaStream_t st)
+cudaError_t launch_eval_sliced(const SampleJob &job, int mode, const LaunchCfg &cfg, cudaStream_t st, int *tile)
 {
     if (job.B <= 0) return cudaSuccess;
-    return mode == EVAL_ABS ? launch_slice<EVAL_ABS>(job, cfg, st) : launch_slice<EVAL_COMPLEX>(job, cfg, st);
+    return mode == EVAL_ABS ? launch_slice<EVAL_ABS>(job, cfg, st, tile)
+                            : launch_slice<EVAL_COMPLEX>(job, cfg, st, tile);
 }
 
 cudaError_t launch_eval(const EvalJob &job, int W, cudaStream_t st)

@@ -85,8 +85,9 @@ struct EvalJob {
 cudaError_t launch_eval(const EvalJob &job, int W, cudaStream_t st);
 
 // |A| or A of one graph over a sliced stream: the job's chunks are the
-// graph's, its rows the parameter vectors, `amp` the output.
-cudaError_t launch_eval_sliced(const SampleJob &job, int mode, const LaunchCfg &cfg, cudaStream_t st);
+// graph's, its rows the parameter vectors, `amp` the output.  *tile: the rows
+// of a tile (SLICE_UNWRITTEN).
+cudaError_t launch_eval_sliced(const SampleJob &job, int mode, const LaunchCfg &cfg, cudaStream_t st, int *tile);
 
 // Bit-packed rows (bit c of a row = byte c/8, bit c%8) <-> one byte per bit.
 cudaError_t launch_unpack_bits(const uint8_t *packed, int64_t rows, int64_t packed_row, int64_t n_cols,

@@ -54,7 +54,6 @@ struct ksim_component {
     int slice_chunks = 0, slice_rows = 0, slice_planes = 0;
     std::vector<int> slice_first;  // per graph: its first chunk (and the end)
     uint32_t *d_status = nullptr;
-    uint32_t *h_status = nullptr;  // page-locked: where a sliced eval call's kernel reports
     cudaStream_t stream = nullptr;
     ksim::DevBuf ws_f, ws_out, ws_aux;
     ksim::LaunchCfg cfg;

@@ -460,7 +460,8 @@ __device__ __forceinline__ uint2 lds64(uint32_t a)
 // CTA's shared memory, parameter rows first, planes at planes_off.  Returns
 // false after a wait timeout (the CTA must then stop using the ring).
 // EVAL: instead of sampling, the job's chunks are one graph's and its rows are
-// whole parameter vectors; |A| (EVAL_ABS) or A (EVAL_COMPLEX) goes to j.amp.
+// whole parameter vectors; |A| (EVAL_ABS) or A (EVAL_COMPLEX) goes to j.amp, or,
+// after a wait timeout, SLICE_UNWRITTEN to the tile's first row.
 template <int S, bool CG = false, int EVAL = -1>
 __device__ __forceinline__ bool slice_tile(const SampleJob &j, const int64_t s0, const int64_t s_end, int shots,
                                            uint8_t *smem, int planes_off, uint64_t *bar, uint32_t &g)
@@ -631,6 +632,7 @@ __device__ __forceinline__ bool slice_tile(const SampleJob &j, const int64_t s0,
         if (__syncthreads_or(!slice_wait(j, &bar[NSLOT], gc & 1u) || !ok)) {
             if (tid == 0) {
                 atomicOr(j.status, (uint32_t)KSIM_FLAG_WAIT_TIMEOUT);
+                if (EVAL >= 0) ((uint64_t *)j.amp)[(EVAL == EVAL_ABS ? 1 : 2) * s0] = SLICE_UNWRITTEN;
                 mbar_wait(&bar[slot], par);
                 mbar_wait(&bar[NSLOT], gc & 1u);
                 if (c + 1 < nch) mbar_wait(&bar[slot ^ 1], ((gc + 1) / NSLOT) & 1u);

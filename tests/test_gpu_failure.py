@@ -117,3 +117,9 @@ def test_eval_reports_a_wait_timeout(cuda_device, oracle_port, call):
     kc.set_wait_limit(0)
     assert same_bits(getattr(kc, call)(3, pv), want)
     assert kc.status() == 0
+    # one tile, one row: its marker alone tells
+    kc.set_wait_limit(1)
+    with pytest.raises(TimeoutError, match="staging wait"):
+        getattr(kc, call)(3, pv[:1])
+    kc.set_wait_limit(0)
+    assert kc.status() == 0 and same_bits(getattr(kc, call)(3, pv[:1]), want[:1])
